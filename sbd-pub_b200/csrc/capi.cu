@@ -272,6 +272,7 @@ int sbd_tpb_sigma(sbd_tpb_handle *h, const double *C, double *sigma, int accumul
   }
   TPB_CHECK(sigma_sep<double>(h, h->d_tmp64, h->d_tmp64b, 0));
   TPB_CUDA(cudaEventSynchronize(h->ev1));
+  TPB_CHECK(ab_rows_check(h));
   TPB_CUDA(cudaEventElapsedTime(&h->last_sigma_ms, h->ev0, h->ev1));
   TPB_CHECK(reorder_sign_apply_f64(h, h->d_tmp64b, h->d_tmp64));
   if (mem == SBD_TPB_DEVICE) {
@@ -304,6 +305,7 @@ int sbd_tpb_sigma_f32(sbd_tpb_handle *h, const float *C, float *sigma, int accum
   }
   TPB_CHECK(sigma_sep<float>(h, h->d_tmp32, h->d_tmp32b, 0));
   TPB_CUDA(cudaEventSynchronize(h->ev1));
+  TPB_CHECK(ab_rows_check(h));
   TPB_CUDA(cudaEventElapsedTime(&h->last_sigma_ms, h->ev0, h->ev1));
   TPB_CHECK(reorder_sign_apply_f32(h, h->d_tmp32b, h->d_tmp32));
   if (mem == SBD_TPB_DEVICE) {
@@ -345,6 +347,7 @@ int sbd_tpb_sigma_device(sbd_tpb_handle *h, const void *C, void *sigma, int dtyp
     TPB_CHECK(sigma_sep<float>(h, (const float *)C, (float *)sigma, accumulate));
   }
   TPB_CUDA(cudaEventSynchronize(h->ev1));
+  TPB_CHECK(ab_rows_check(h));
   TPB_CUDA(cudaEventElapsedTime(&h->last_sigma_ms, h->ev0, h->ev1));
   return SBD_TPB_OK;
 }

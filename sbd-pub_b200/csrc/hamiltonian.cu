@@ -236,6 +236,7 @@ void free_device_problem(sbd_tpb_handle *h) {
   free_dev(h->ab.Vlo);
   free_dev(h->ab.err);
   h->ab = ABDense();
+  ab_rows_free(h);
   pool_clear(h);
   free_dev(h->d_partials);
   h->partials_cap = 0;

@@ -1134,9 +1134,11 @@ int launch_ab_sparse(sbd_tpb_handle *h, const T *C, T *sigma, double scale = 1.0
 template <typename T>
 int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, double shift) {
   const uint32_t na = (uint32_t)h->astr.size(), nb = (uint32_t)h->bstr.size();
-  // dense alpha-beta path only where the contraction runs on the tensor cores (FP32 vectors): in
-  // FP64 the shared-memory sparse kernel is faster even at full-CI connectivity (norb=12 FCI:
-  // 1.5 ms against 3.4 ms for the CUDA-core gather/contract/scatter)
+  // Alpha-beta term: densely connected sets take one product per alpha row (ab_rows.cu; when, see
+  // ab_rows_prepare), except small FP32 problems, whose gather / contraction / scatter on tcgen05 is
+  // still ahead at full-CI connectivity (norb=12 FCI symmetric 0.341 against 0.354 ms); in FP64 the
+  // CUDA-core form of that path loses to both others (3.4 ms there).  Sparse singles take the direct
+  // kernel.
   const bool dense_ab = h->ab.enabled && sizeof(T) == 4 && h->ab.tc_ready;
   const size_t n = h->ndet();
   if (h->ct_bytes < n * sizeof(T)) {
@@ -1147,7 +1149,9 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
     h->ct_bytes = n * sizeof(double);
   }
   T *CT = reinterpret_cast<T *>(h->d_ct);
-  TPB_CHECK(prepare_sigma_meta(h, !dense_ab));
+  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h));
+  const bool rows_ab = h->abr.ready && !dense_ab;
+  TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab));
   // per-pair Coulomb sums of the singles over the other spin's strings (built once per problem)
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   TPB_CHECK(build_coulomb_table(h, h->pb, h->d_astr, na));
@@ -1205,7 +1209,9 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
   bb.max_s = h->blk_max[3];
   TPB_CHECK((launch_block<T, false>(h, bb, CT, sigma, nullptr)));
   TPB_CUDA(cudaEventRecord(h->ev_k[1], h->stream));
-  if (dense_ab) {
+  if (rows_ab) {
+    TPB_CHECK(ab_rows_apply<T>(h, C, sigma, false));
+  } else if (dense_ab) {
     TPB_CHECK(ab_dense_apply<T>(h, C, sigma));
   } else {
     TPB_CHECK(launch_ab_sparse<T>(h, C, sigma));
@@ -1232,7 +1238,9 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
   if (na != nb || h->astr != h->bstr)
     return fail(SBD_TPB_ERR_STATE, "symmetric sigma needs identical alpha and beta strings");
   const bool dense_ab = h->ab.enabled && sizeof(T) == 4 && h->ab.tc_ready;
-  TPB_CHECK(prepare_sigma_meta(h, !dense_ab));
+  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h));
+  const bool rows_ab = h->abr.ready && !dense_ab;
+  TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab));
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   BlockArgs ba{};
   ba.s_off = h->ta_s.off;
@@ -1261,7 +1269,9 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
   TPB_CUDA(cudaEventRecord(h->ev0, h->stream));
   TPB_CHECK(launch_block_sym<T>(h, ba, C, sigma));
   TPB_CUDA(cudaEventRecord(h->ev_k[0], h->stream));
-  if (dense_ab) {
+  if (rows_ab) {
+    TPB_CHECK(ab_rows_apply<T>(h, C, sigma, true));
+  } else if (dense_ab) {
     TPB_CHECK(ab_dense_apply<T>(h, C, sigma, 0.5));
   } else {
     TPB_CHECK(launch_ab_sparse<T>(h, C, sigma, 1.0, true));

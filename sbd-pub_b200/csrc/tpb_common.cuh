@@ -122,6 +122,20 @@ struct ABDense {
   int *err = nullptr;             // bounded-wait status of the tensor-core kernel
 };
 
+// Alpha-beta term as one product per alpha row (ab_rows.cu): the beta singles as a program over
+// blocks of ket columns, and the alpha singles in the order the symmetric form needs.
+struct ABRows {
+  bool tried = false, ready = false;
+  uint32_t *rows = nullptr;                      // alpha rows with singles, most singles first
+  uint2 *ent = nullptr;                          // alpha singles (ket, +-(pair + 1))
+  int32_t *pair_m = nullptr, *m_pair = nullptr;  // pair <-> row of the product
+  uint4 *hdr = nullptr;
+  unsigned char *prog = nullptr;
+  int M = 0, passes = 0, bpp = 0;
+  uint32_t nrows = 0, nchunks = 0, kcap = 0, prog_cap = 0;
+  int *err = nullptr;  // status of the kernel's bounded waits (pinned host memory it writes to)
+};
+
 }  // namespace sbdtpb
 
 struct sbd_tpb_handle {
@@ -163,6 +177,7 @@ struct sbd_tpb_handle {
   sbdtpb::ExTable ta_s, ta_d, tb_s, tb_d;
   sbdtpb::SigmaProg pa, pb;
   sbdtpb::ABDense ab;
+  sbdtpb::ABRows abr;
 
   // scratch
   double *d_partials = nullptr;  // reduction partial sums
@@ -240,6 +255,12 @@ int ab_dense_setup(sbd_tpb_handle *h, int enable);
 bool ab_dense_worthwhile(sbd_tpb_handle *h);
 template <typename T>
 int ab_dense_apply(sbd_tpb_handle *h, const T *C, T *sigma, double scale = 1.0);
+// ab_rows.cu: alpha-beta term of densely connected sets, one tensor-core product per alpha row
+int ab_rows_prepare(sbd_tpb_handle *h);
+void ab_rows_free(sbd_tpb_handle *h);
+int ab_rows_check(sbd_tpb_handle *h);  // status of the launches before the last synchronisation
+template <typename T>
+int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym, double scale = 1.0);
 // vecops.cu
 int ensure_partials(sbd_tpb_handle *h, size_t n);
 template <typename T>

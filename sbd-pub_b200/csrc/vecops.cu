@@ -1205,7 +1205,7 @@ static int finish_reduce(sbd_tpb_handle *h, int nvals, double *host_out, int nbl
   TPB_CUDA(cudaMemcpyAsync(host_out, d_out, sizeof(double) * nvals, cudaMemcpyDeviceToHost,
                            h->stream));
   TPB_CUDA(cudaStreamSynchronize(h->stream));
-  return SBD_TPB_OK;
+  return ab_rows_check(h);
 }
 
 // compile-time subspace size from a runtime one (1 .. kMaxVec)
@@ -1355,6 +1355,7 @@ const double *fetch_scalars(sbd_tpb_handle *h, int count) {
     fail(SBD_TPB_ERR_CUDA, "fetching reduction results failed");
     return nullptr;
   }
+  if (ab_rows_check(h) != SBD_TPB_OK) return nullptr;
   return h->h_scal;
 }
 

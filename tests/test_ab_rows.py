@@ -1,0 +1,94 @@
+"""The alpha-beta term of densely connected string sets (csrc/ab_rows.cu: one product per alpha row and
+a gather over the beta singles) against the oracle, at the sizes where its tiling can go wrong.
+
+Sets: n strings of lowest orbital-index sum with noise, so that they hold tens of singles each.  Column
+steps are 32 wide, rows of the product come in blocks of 8 (one pass up to 24 blocks), singles in groups
+of 64, and a sigma row that does not fit shared memory is added to in place.
+"""
+import itertools
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(norb, n, count, seed):
+    idx = np.array(list(itertools.combinations(range(norb), n)), np.int64)
+    score = idx.sum(axis=1) + 2.0 * np.random.default_rng(seed).gumbel(size=len(idx))
+    score[0] = -np.inf
+    keep = np.argsort(score, kind="stable")[:count]
+    return np.sort((np.int64(1) << idx[keep]).sum(axis=1).astype(np.uint64))
+
+
+CASES = {
+    # norb, (alpha electrons, strings), (beta electrons, strings): what is at its edge
+    "full8": (8, (4, 70), (4, 70)),            # 28 pairs: the last block of 8 rows half empty
+    "full7_33": (7, (3, 35), (2, 21)),         # fewer columns than one step
+    "chunk_exact": (12, (4, 256), (4, 256)),   # whole steps, last one full
+    "chunk_plus1": (12, (4, 257), (4, 257)),   # last step one column
+    "two_groups": (18, (7, 600), (7, 600)),    # up to 77 singles in a row: two groups of at most 64
+    "two_passes": (24, (5, 401), (4, 333)),    # up to 276 pairs: two passes over the rows of the product
+    "one_row": (10, (5, 2), (5, 252)),         # rows with a single single
+    "wide": (18, (7, 24), (7, 15001)),         # a sigma row longer than shared memory holds in FP64
+}
+
+
+def _problem(name):
+    import synth
+    from sbd_tpb import Problem
+    norb, (ea, na), (eb, nb) = CASES[name]
+    h1, eri, core = synth.synthetic_hamiltonian(norb, seed=5)
+    a = _dense(norb, ea, na, 1)
+    b = a.copy() if (ea, na) == (eb, nb) else _dense(norb, eb, nb, 2)
+    return Problem(norb=norb, nelec=ea + eb, core=core, h1=h1, eri_packed=eri, astr=a, bstr=b)
+
+
+def _oracle_rows(prob, x, rows):
+    import pyoracle
+    ham = pyoracle.Hamiltonian.from_arrays(prob.norb, prob.nelec, prob.core, prob.h1, prob.eri_packed)
+    return pyoracle.System(ham, prob.astr, prob.bstr).sigma_rows(rows, x)
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_alpha_beta_rows_against_oracle(name):
+    import sbd_tpb
+    prob = _problem(name)
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    rng = np.random.default_rng(7)
+    x = rng.normal(size=prob.ndet)
+    rows = np.sort(rng.choice(prob.ndet, size=min(300, prob.ndet), replace=False)).astype(np.uint64)
+    ref = _oracle_rows(prob, x, rows)
+    out = h.sigma(x)
+    assert np.array_equal(out, h.sigma(x))  # one owner per element: the same bits again
+    scale = float(np.max(np.abs(ref)))
+    # FP64 sums of the same terms in another order
+    assert float(np.max(np.abs(out[rows] - ref))) <= 1e-12 * scale
+    # FP32: vectors and results rounded to FP32, 2^-24 a value over a few thousand terms of random sign
+    out32 = h.sigma(x.astype(np.float32)).astype(np.float64)
+    assert float(np.max(np.abs(out32[rows] - ref))) <= 2e-6 * scale
+    h.close()
+
+
+@pytest.mark.parametrize("name", [n for n in sorted(CASES) if CASES[n][1] == CASES[n][2]])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_alpha_beta_rows_symmetric_half(name, dtype):
+    """The symmetric form adds only the half of the terms whose transposes are the other half."""
+    import torch
+
+    import sbd_tpb
+    prob = _problem(name)
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    n = len(prob.astr)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = torch.randn(n, n, dtype=torch.float64, device="cuda", generator=g)
+    x = (r + r.T).to(getattr(torch, dtype)).reshape(-1).contiguous()
+    ref, out = torch.zeros_like(x), torch.full_like(x, float("nan"))
+    torch.cuda.synchronize()  # the library runs on a stream of its own
+    h.sigma_device(x, ref)
+    h.sigma_device(x, out, symmetric=True)
+    err = float((out.double() - ref.double()).abs().max()) / float(ref.double().abs().max())
+    assert err <= (1e-13 if dtype == "float64" else 3e-6), err
+    h.close()
