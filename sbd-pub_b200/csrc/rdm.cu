@@ -284,6 +284,43 @@ __global__ void __launch_bounds__(kRdmThreads)
   for (int i = threadIdx.x; i < L2; i += blockDim.x) X[(size_t)e * L2 + i] = accs[i];
 }
 
+// Sums over the singles that share a label (cr, an), one CTA per label (seg[b] .. seg[b + 1] of the
+// list ord: +-(entry + 1) with the single's sign), always in list order, so they repeat bit for bit.
+//   rdm_label_sum_kernel     out[b][k] = sum +-X[entry][k]
+//   rdm_label_occ_kernel     out[b][j] = sum +-T0[entry] for the entries whose bra string holds j
+// The host used to fetch X (one row of L^2 per alpha single: 107 MB at 18 orbitals, 1,387 strings) and
+// add up its rows, and to place every single's own sums; the label sums are L^2 x L^2 numbers.  Bound by
+// reading X once; whole call there 150 -> 30 ms (of which 12 ms are the pair kernels).
+__global__ void __launch_bounds__(kRdmThreads)
+    rdm_label_sum_kernel(const double *__restrict__ X, int width, const uint32_t *__restrict__ seg,
+                         const int32_t *__restrict__ ord, double *__restrict__ out) {
+  const uint32_t b0 = seg[blockIdx.x], b1 = seg[blockIdx.x + 1];
+  for (int k = blockIdx.y * kRdmThreads + threadIdx.x; k < width; k += gridDim.y * kRdmThreads) {
+    double s = 0.0;
+#pragma unroll 8
+    for (uint32_t i = b0; i < b1; i++) {
+      const int32_t o = __ldg(&ord[i]);
+      const double v = X[(size_t)((o > 0 ? o : -o) - 1) * width + k];
+      s += o > 0 ? v : -v;
+    }
+    out[(size_t)blockIdx.x * width + k] = s;
+  }
+}
+
+__global__ void __launch_bounds__(64)
+    rdm_label_occ_kernel(const double *__restrict__ T0, const uint64_t *__restrict__ bra, const uint32_t *__restrict__ seg,
+                         const int32_t *__restrict__ ord, double *__restrict__ out) {
+  const uint32_t b0 = seg[blockIdx.x], b1 = seg[blockIdx.x + 1];
+  double s = 0.0;
+#pragma unroll 4
+  for (uint32_t i = b0; i < b1; i++) {
+    const int32_t o = __ldg(&ord[i]);
+    const double v = T0[(o > 0 ? o : -o) - 1];
+    if ((bra[i] >> threadIdx.x) & 1) s += o > 0 ? v : -v;
+  }
+  out[(size_t)blockIdx.x * 64 + threadIdx.x] = s;
+}
+
 struct HostTable {
   std::vector<uint32_t> off, ket, lab;
 };
@@ -443,58 +480,129 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
       transpose_kernel<<<grid, block, 0, h->stream>>>(W, d_WT, na, nb);
       TPB_LAUNCHED(h);
     }
-    std::vector<double> T0, Tq;
+    std::vector<double> T0;
+    // the singles of one spin by their label: seg/ord as the kernels take them, and each one's bra
+    struct Labels {
+      std::vector<int> pair;  // an * L + cr of each label
+      uint32_t *seg = nullptr;
+      int32_t *ord = nullptr;
+      uint64_t *bra = nullptr;
+      ~Labels() {
+        cudaFree(seg);
+        cudaFree(ord);
+        cudaFree(bra);
+      }
+    };
+    auto labels = [&](const HostTable &ht, const std::vector<uint64_t> &str, Labels &lb) -> int {
+      std::vector<uint32_t> count((size_t)L * L + 1, 0), seg;
+      for (uint32_t l : ht.lab) count[((l >> 8) & 0xff) * L + (l & 0xff)]++;
+      std::vector<uint32_t> at((size_t)L * L);
+      uint32_t w = 0;
+      for (int p = 0; p < L * L; p++) {
+        at[p] = w;
+        if (count[p]) {
+          lb.pair.push_back(p);
+          seg.push_back(w);
+        }
+        w += count[p];
+      }
+      seg.push_back(w);
+      std::vector<int32_t> ord(w);
+      std::vector<uint64_t> bra(w);
+      for (size_t i = 0; i < str.size(); i++)
+        for (uint32_t e = ht.off[i]; e < ht.off[i + 1]; e++) {
+          const int cr = ht.lab[e] & 0xff, an = (ht.lab[e] >> 8) & 0xff;
+          const uint32_t t = at[an * L + cr]++;
+          ord[t] = single_sign(str[i], cr, an) > 0 ? (int32_t)e + 1 : -((int32_t)e + 1);
+          bra[t] = str[i];
+        }
+      TPB_CUDA(cudaMalloc(&lb.seg, sizeof(uint32_t) * seg.size()));
+      TPB_CUDA(cudaMalloc(&lb.ord, sizeof(int32_t) * std::max<size_t>(1, w)));
+      TPB_CUDA(cudaMalloc(&lb.bra, sizeof(uint64_t) * std::max<size_t>(1, w)));
+      TPB_CUDA(cudaMemcpy(lb.seg, seg.data(), sizeof(uint32_t) * seg.size(), cudaMemcpyHostToDevice));
+      TPB_CUDA(cudaMemcpy(lb.ord, ord.data(), sizeof(int32_t) * w, cudaMemcpyHostToDevice));
+      TPB_CUDA(cudaMemcpy(lb.bra, bra.data(), sizeof(uint64_t) * w, cudaMemcpyHostToDevice));
+      return SBD_TPB_OK;
+    };
+    Labels la, lbeta;
+    // sums over the labels of lb: label_sum(X, width, ...) of the rows of X, or (X == d_T0, width 64)
+    // the occupation-resolved sums of rdm_label_occ_kernel
+    auto label_sums = [&](const Labels &lb, const double *X, int width, bool occ, std::vector<double> &out) -> int {
+      const unsigned nl = (unsigned)lb.pair.size();
+      out.resize((size_t)nl * width);
+      if (!nl) return SBD_TPB_OK;
+      double *d_out = nullptr;
+      TPB_CUDA(cudaMalloc(&d_out, sizeof(double) * out.size()));
+      if (occ) {
+        rdm_label_occ_kernel<<<nl, 64, 0, h->stream>>>(X, lb.bra, lb.seg, lb.ord, d_out);
+      } else {
+        dim3 grid(nl, (unsigned)((width + kRdmThreads - 1) / kRdmThreads));
+        rdm_label_sum_kernel<<<grid, kRdmThreads, 0, h->stream>>>(X, width, lb.seg, lb.ord, d_out);
+      }
+      h->launches++;
+      cudaError_t e = cudaGetLastError();
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(out.data(), d_out, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, h->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+      cudaFree(d_out);
+      if (e != cudaSuccess) return fail(SBD_TPB_ERR_CUDA, std::string("rdm label sums: ") + cudaGetErrorString(e));
+      return SBD_TPB_OK;
+    };
     // same-spin pairs; s = 0 alpha (rows of W), 1 beta (rows of W^T)
+    std::vector<double> D;  // doubles: [i0 L + j0][a0 L + b0]
     auto run_pairs = [&](int s, const double *X, uint32_t nrow, uint32_t ncol, const ExTable &t,
                          const HostTable &ht, const uint64_t *d_other, bool single) -> int {
       if (t.nnz == 0) return SBD_TPB_OK;
       rdm_pair_kernel<<<nrow, kRdmThreads, 0, h->stream>>>(X, ncol, t.off, t.ket, d_other, L, d_T0,
                                                          single ? d_Tq : nullptr);
       TPB_LAUNCHED(h);
+      const std::vector<uint64_t> &str = s == 0 ? h->astr : h->bstr;
+      if (single) {
+        const Labels &lb = s == 0 ? la : lbeta;
+        std::vector<double> own, other;  // with a number operator of the same spin, of the other
+        TPB_CHECK(label_sums(lb, d_T0, 64, true, own));
+        TPB_CHECK(label_sums(lb, d_Tq, L, false, other));
+        for (size_t k = 0; k < lb.pair.size(); k++) {
+          const int cr = lb.pair[k] % L, an = lb.pair[k] / L;
+          R.g(s, cr, an) += own[k * 64 + cr];  // every bra of the label holds cr
+          for (int j = 0; j < L; j++) {
+            if (j != cr && own[k * 64 + j] != 0.0) R.single_with_number(s, cr, an, s, j, own[k * 64 + j]);
+            if (other[k * L + j] != 0.0) R.single_with_number(s, cr, an, 1 - s, j, other[k * L + j]);
+          }
+        }
+        return SBD_TPB_OK;
+      }
       T0.resize(t.nnz);
       TPB_CUDA(cudaMemcpyAsync(T0.data(), d_T0, sizeof(double) * t.nnz, cudaMemcpyDeviceToHost, h->stream));
-      if (single) {
-        Tq.resize(t.nnz * L);
-        TPB_CUDA(cudaMemcpyAsync(Tq.data(), d_Tq, sizeof(double) * t.nnz * L, cudaMemcpyDeviceToHost, h->stream));
-      }
       TPB_CUDA(cudaStreamSynchronize(h->stream));
-      const std::vector<uint64_t> &str = s == 0 ? h->astr : h->bstr;
-      const int o = 1 - s;
+      D.assign(R.L4, 0.0);
       for (uint32_t i = 0; i < nrow; i++) {
         const uint64_t I = str[i];
         for (uint32_t e = ht.off[i]; e < ht.off[i + 1]; e++) {
           const uint32_t lab = ht.lab[e];
-          if (single) {
-            const int cr = lab & 0xff, an = (lab >> 8) & 0xff;
-            const double x = single_sign(I, cr, an) * T0[e];
-            R.g(s, cr, an) += x;
-            uint64_t occ = I & ~(1ull << cr);
-            while (occ) {
-              const int j = __builtin_ctzll(occ);
-              R.single_with_number(s, cr, an, s, j, x);
-              occ &= occ - 1;
-            }
-            const double sg = single_sign(I, cr, an);
-            for (int j = 0; j < L; j++) {
-              const double y = sg * Tq[(size_t)e * L + j];
-              if (y != 0.0) R.single_with_number(s, cr, an, o, j, y);
-            }
-          } else {
-            const int i0 = lab & 0xff, j0 = (lab >> 8) & 0xff, a0 = (lab >> 16) & 0xff,
-                      b0 = (lab >> 24) & 0xff;
-            const double x = double_sign(I, i0, j0, a0, b0) * T0[e];
-            // <c+_{i0} c+_{j0} c_{b0} c_{a0}> = sign, and the three reorderings
-            R.G(s, s, i0, j0, a0, b0) += x;
-            R.G(s, s, j0, i0, b0, a0) += x;
-            R.G(s, s, i0, j0, b0, a0) -= x;
-            R.G(s, s, j0, i0, a0, b0) -= x;
-          }
+          const int i0 = lab & 0xff, j0 = (lab >> 8) & 0xff, a0 = (lab >> 16) & 0xff, b0 = (lab >> 24) & 0xff;
+          D[((size_t)i0 * L + j0) * R.L2 + (size_t)a0 * L + b0] += double_sign(I, i0, j0, a0, b0) * T0[e];
         }
       }
+      for (int i0 = 0; i0 < L; i0++)
+        for (int j0 = i0 + 1; j0 < L; j0++) {
+          const double *d = D.data() + ((size_t)i0 * L + j0) * R.L2;
+          for (int a0 = 0; a0 < L; a0++)
+            for (int b0 = a0 + 1; b0 < L; b0++) {
+              const double x = d[(size_t)a0 * L + b0];
+              if (x == 0.0) continue;
+              // <c+_{i0} c+_{j0} c_{b0} c_{a0}> = sign, and the three reorderings
+              R.G(s, s, i0, j0, a0, b0) += x;
+              R.G(s, s, j0, i0, b0, a0) += x;
+              R.G(s, s, i0, j0, b0, a0) -= x;
+              R.G(s, s, j0, i0, a0, b0) -= x;
+            }
+        }
       return SBD_TPB_OK;
     };
     int rc = SBD_TPB_OK;
-    if ((rc = run_pairs(0, W, na, nb, h->ta_s, as, h->d_bstr, true)) == SBD_TPB_OK &&
+    if ((rc = labels(as, h->astr, la)) == SBD_TPB_OK && (rc = labels(bs, h->bstr, lbeta)) == SBD_TPB_OK &&
+        (rc = run_pairs(0, W, na, nb, h->ta_s, as, h->d_bstr, true)) == SBD_TPB_OK &&
         (rc = run_pairs(0, W, na, nb, h->ta_d, ad, h->d_bstr, false)) == SBD_TPB_OK &&
         (rc = run_pairs(1, d_WT, nb, na, h->tb_s, bs, h->d_astr, true)) == SBD_TPB_OK &&
         (rc = run_pairs(1, d_WT, nb, na, h->tb_d, bd, h->d_astr, false)) == SBD_TPB_OK) {
@@ -531,22 +639,21 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
       rdm_mixed_kernel<<<(unsigned)h->ta_s.nnz, kRdmThreads, sizeof(double) * L2, h->stream>>>(
           W, nb, d_abra, h->ta_s.ket, d_bbra, h->tb_s.ket, d_blab, (uint32_t)h->tb_s.nnz, L2, d_X);
       TPB_LAUNCHED(h);
-      std::vector<double> X(h->ta_s.nnz * (size_t)L2);
-      TPB_CUDA(cudaMemcpyAsync(X.data(), d_X, sizeof(double) * X.size(), cudaMemcpyDeviceToHost, h->stream));
-      TPB_CUDA(cudaStreamSynchronize(h->stream));
+      // summed over the alpha singles of each label: one row of L^2 per (an, cr)
+      std::vector<double> X;
+      const int src = label_sums(la, d_X, L2, false, X);
       cudaFree(d_abra);
       cudaFree(d_bbra);
       cudaFree(d_blab);
       cudaFree(d_X);
-      for (uint32_t i = 0; i < na; i++)
-        for (uint32_t e = as.off[i]; e < as.off[i + 1]; e++) {
-          const int cra = as.lab[e] & 0xff, ana = (as.lab[e] >> 8) & 0xff;
-          const double sa = single_sign(h->astr[i], cra, ana);
-          const double *xr = X.data() + (size_t)e * L2;
+      TPB_CHECK(src);
+      for (size_t k = 0; k < la.pair.size(); k++) {
+          const int cra = la.pair[k] % L, ana = la.pair[k] / L;
+          const double *xr = X.data() + k * (size_t)L2;
           for (int rs = 0; rs < L2; rs++) {
             if (xr[rs] == 0.0) continue;
             const int crb = rs / L, anb = rs % L;
-            const double x = sa * xr[rs];
+            const double x = xr[rs];
             // placement of TwoDiffCorrelation for an alpha-single x beta-single pair
             // (basic/correlation.h:191-231): spin-orbitals ordered I<J (bra), A<B (ket); the
             // value is the separated-convention sign sa*sb times W_bra W_ket in either branch
