@@ -56,6 +56,23 @@ int ensure_tmp32(sbd_tpb_handle *h) {
   return SBD_TPB_OK;
 }
 
+// Device vectors are usually written by work the caller queued on the legacy default stream (where
+// torch and plain launches go), which the handle's non-blocking stream does not wait for by itself: a
+// sigma called right behind the kernel that makes its input read it half written.  The wait is on the
+// device, for what is queued so far; while a stream that blocks on the legacy one is capturing (the
+// query says so without disturbing the capture) ordering stays with the caller, as it does for
+// vectors made on other streams.
+int wait_for_caller(sbd_tpb_handle *h) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return SBD_TPB_OK;
+  }
+  TPB_CUDA(cudaEventRecord(h->ev_in, cudaStreamLegacy));
+  TPB_CUDA(cudaStreamWaitEvent(h->stream, h->ev_in, 0));
+  return SBD_TPB_OK;
+}
+
 void free_tmps(sbd_tpb_handle *h) {
   for (double **p : {&h->d_tmp64, &h->d_tmp64b})
     if (*p) {
@@ -112,6 +129,7 @@ int sbd_tpb_create(int device, sbd_tpb_handle **out) {
   bool ev_ok = cudaEventCreate(&h->ev0) == cudaSuccess && cudaEventCreate(&h->ev1) == cudaSuccess;
   for (cudaEvent_t &e : h->ev_k) ev_ok = ev_ok && cudaEventCreate(&e) == cudaSuccess;
   for (cudaEvent_t &e : h->ev_co) ev_ok = ev_ok && cudaEventCreate(&e) == cudaSuccess;
+  ev_ok = ev_ok && cudaEventCreateWithFlags(&h->ev_in, cudaEventDisableTiming) == cudaSuccess;
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess || !ev_ok) {
     delete h;
     return fail(SBD_TPB_ERR_CUDA, "stream/event creation failed");
@@ -131,6 +149,7 @@ int sbd_tpb_destroy(sbd_tpb_handle *h) {
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : h->ev_co)
     if (e) cudaEventDestroy(e);
+  if (h->ev_in) cudaEventDestroy(h->ev_in);
   if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -265,6 +284,7 @@ int sbd_tpb_sigma(sbd_tpb_handle *h, const double *C, double *sigma, int accumul
   TPB_CHECK(ensure_tmp64(h));
   // reference convention in, separated convention inside: x = D C
   if (mem == SBD_TPB_DEVICE) {
+    TPB_CHECK(wait_for_caller(h));
     TPB_CHECK(reorder_sign_apply_f64(h, C, h->d_tmp64));
   } else {
     TPB_CUDA(cudaMemcpyAsync(h->d_tmp64b, C, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
@@ -298,6 +318,7 @@ int sbd_tpb_sigma_f32(sbd_tpb_handle *h, const float *C, float *sigma, int accum
   const size_t n = h->ndet();
   TPB_CHECK(ensure_tmp32(h));
   if (mem == SBD_TPB_DEVICE) {
+    TPB_CHECK(wait_for_caller(h));
     TPB_CHECK(reorder_sign_apply_f32(h, C, h->d_tmp32));
   } else {
     TPB_CUDA(cudaMemcpyAsync(h->d_tmp32b, C, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream));
@@ -337,6 +358,7 @@ int sbd_tpb_sigma_device(sbd_tpb_handle *h, const void *C, void *sigma, int dtyp
   if (convention != 1 && convention != 2) return fail(SBD_TPB_ERR_INVALID, "convention must be 0, 1 or 2");
   // the passes read C while they write sigma
   if (C == sigma) return fail(SBD_TPB_ERR_INVALID, "sigma_device: C and sigma must be distinct buffers");
+  TPB_CHECK(wait_for_caller(h));
   if (convention == 2) {
     if (accumulate) return fail(SBD_TPB_ERR_INVALID, "sigma_device: convention 2 does not accumulate");
     if (dtype == 0) TPB_CHECK(sigma_sep_sym<double>(h, (const double *)C, (double *)sigma, 0.0));

@@ -146,6 +146,7 @@ struct sbd_tpb_handle {
   uint64_t launches = 0;
   float last_sigma_ms = 0.f;
   int sigma_kernels = 0;  // kernels timed in the last sigma (ev0, ev_k[0..], ev1)
+  cudaEvent_t ev_in = nullptr;  // work queued by the caller before a call on device vectors
   cudaEvent_t ev_co[2] = {nullptr, nullptr};  // around the weight pass of the last carry-over
   float last_carryover_ms[2] = {0.f, 0.f};    // weight pass, whole call
   float last_parse_ms = 0.f;                   // last string-file parse (copy, parse, sort)
