@@ -175,7 +175,11 @@ __global__ void __launch_bounds__(kBlkThreads, M)
   const int L = a.L, L2 = L * L;
   const int nr = (int)min((uint32_t)kBlkRows, a.nrows - r0);
   const int grp = threadIdx.x / TC;                                  // row group of this thread
-  const uint32_t cbase = slab * W + (threadIdx.x % TC) * VW;         // first of its VW columns
+  // its VW columns, cbase + i * kStep: neighbours for 16-byte accesses; with scalar accesses TC apart,
+  // so that each access of a warp is one contiguous run (28 orbitals, 9,999 strings: FP32 one-pass 2.41
+  // -> 1.71 ms, general alpha pass FP32 2.78 -> 2.21, FP64 3.18 -> 2.77; the beta passes within 4 %)
+  constexpr uint32_t kStep = kVec ? 1 : TC;
+  const uint32_t cbase = slab * W + (threadIdx.x % TC) * (kVec ? VW : 1);
 
   // stage the block's table entries
   const uint32_t dlo = __ldg(&a.d_off[r0]), dhi = __ldg(&a.d_off[r0 + nr]);
@@ -195,8 +199,8 @@ __global__ void __launch_bounds__(kBlkThreads, M)
   uint64_t cstr[VW];
 #pragma unroll
   for (int i = 0; i < VW; i++) {
-    ok[i] = cbase + i < ncols;
-    cstr[i] = ok[i] ? __ldg(&a.col_str[cbase + i]) : 0ull;
+    ok[i] = cbase + i * kStep < ncols;
+    cstr[i] = ok[i] ? __ldg(&a.col_str[cbase + i * kStep]) : 0ull;
   }
   const bool any = ok[0];
   const bool full = ok[VW - 1];
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(kBlkThreads, M)
         x.load(xr);
       } else {
 #pragma unroll
-        for (int i = 0; i < VW; i++) x.v[i] = ok[i] ? __ldg(xr + i) : T(0);
+        for (int i = 0; i < VW; i++) x.v[i] = ok[i] ? __ldg(xr + i * kStep) : T(0);
       }
 #pragma unroll
       for (int i = 0; i < VW; i++) acc[r][i] = madd(acc[r][i], v, x.v[i]);
@@ -260,7 +264,7 @@ __global__ void __launch_bounds__(kBlkThreads, M)
 #pragma unroll
       for (int i = 0; i < VW; i++) {
         if (!ok[i]) continue;
-        const uint32_t c = cbase + i;
+        const uint32_t c = cbase + i * kStep;
         double o = 0.0;
         if (jr) {
           o = __ldg(&jr[c]);
@@ -300,9 +304,9 @@ __global__ void __launch_bounds__(kBlkThreads, M)
       } else {
 #pragma unroll
         for (int i = 0; i < VW; i++) {
-          xo.v[i] = ok[i] ? __ldg(X + idx + i) : T(0);
-          hv.v[i] = ok[i] ? __ldg(hsrc + idx + i) : T(0);
-          ov.v[i] = (ok[i] && a.accumulate) ? out[idx + i] : T(0);
+          xo.v[i] = ok[i] ? __ldg(X + idx + i * kStep) : T(0);
+          hv.v[i] = ok[i] ? __ldg(hsrc + idx + i * kStep) : T(0);
+          ov.v[i] = (ok[i] && a.accumulate) ? out[idx + i * kStep] : T(0);
         }
       }
 #pragma unroll
@@ -323,7 +327,7 @@ __global__ void __launch_bounds__(kBlkThreads, M)
       } else {
 #pragma unroll
         for (int i = 0; i < VW; i++)
-          if (ok[i]) out[idx + i] = ov.v[i];
+          if (ok[i]) out[idx + i * kStep] = ov.v[i];
       }
     }
   }
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(kBlkThreads, M)
 #pragma unroll
   for (int i = 0; i < VW; i++) {
     if (!ok[i]) continue;
-    const size_t o = (size_t)(cbase + i) * a.nrows + r0 + rlo;
+    const size_t o = (size_t)(cbase + i * kStep) * a.nrows + r0 + rlo;
     if constexpr (kRuns) {
       if (vec_out) {
 #pragma unroll
@@ -889,6 +893,17 @@ int launch_pass_cm(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T
   return SBD_TPB_OK;
 }
 
+// Small problems (fewer than 8,192 determinants per SM): the usual tiles (8 rows x 512 FP32 / 256 FP64
+// columns, 4 rows a thread) do not fill the GPU and each thread's chain of gathers is the time.  One
+// row per thread then: an eighth of the columns per CTA, a quarter of the chain.  Same bits.  ms per pass,
+// usual -> one row: 8-orbital full CI FP64 0.028 -> 0.015; 12-orbital 0.196 -> 0.155, FP32 0.130 -> 0.106;
+// 24 orbitals, 1,001 strings FP32 0.046 -> 0.030, 401 dense strings FP64 0.194 -> 0.067; 18 orbitals, 642
+// strings FP64 0.301 -> 0.104.  Above the line it wins less or loses: 18 orbitals, 1,387 strings FP64
+// 0.86 -> 0.81, 24 orbitals, 4,000 strings 0.53 -> 0.67.
+inline bool small_problem(const sbd_tpb_handle *h, size_t nrows, size_t ncols) {
+  return nrows * ncols < 8192 * (size_t)h->num_sms;
+}
+
 // Launch shapes of the general passes.  16-byte rows without the alpha-single x beta-single terms
 // take sigma_pass_cm_kernel; from a sweep (CUDA events, ms at 4e8 / 1e8 determinants, row groups /
 // CTAs per SM / column groups, "os": own values parked in shared memory), all giving the same bits:
@@ -902,6 +917,8 @@ int launch_pass_cm(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T
 template <typename T, bool kAlpha>
 int launch_block(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T *XT) {
   constexpr int VW = 16 / sizeof(T);
+  if (!ba.do_ab && small_problem(h, ba.nrows, ba.ncols))
+    return launch_block_cfg<T, kAlpha, 8, 8>(h, ba, X, out, XT);
   const bool rows16 = (ba.ncols % VW) == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0 && (!XT || reinterpret_cast<uintptr_t>(XT) % 16 == 0);
   if (rows16 && !ba.do_ab) {
@@ -953,6 +970,7 @@ int launch_sym_cm(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out) {
 // rows that are not 16-byte aligned) took FP32 2.78 / 1.22 and FP64 4.83 / 2.08 at its best shape.
 template <typename T>
 int launch_block_sym(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out) {
+  if (small_problem(h, ba.nrows, ba.ncols)) return launch_block_cfg<T, true, 8, 8, false, true>(h, ba, X, out, nullptr);
   const bool rows16 = (ba.ncols % (16 / sizeof(T))) == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0;
   if (!rows16) return launch_block_cfg<T, true, 2, 8, false, true>(h, ba, X, out, nullptr);
