@@ -125,6 +125,10 @@ void free_prog(SigmaProg &p) {
   free_dev(p.s_pair);
   free_dev(p.d_val);
   free_dev(p.d_valf);
+  free_dev(p.u_off);
+  free_dev(p.u_ket);
+  free_dev(p.u_val);
+  free_dev(p.u_valf);
   p = SigmaProg();
 }
 

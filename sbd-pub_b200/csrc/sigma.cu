@@ -26,6 +26,7 @@ namespace {
 
 constexpr int kBlkRows = 8;  // bra rows per CTA
 constexpr int kBlkThreads = 128;
+constexpr double kUnionReuse = 1.5;  // doubles per distinct ket of a row block from which the union passes run
 // Thread mapping of a CTA per element type and pass: the 128 threads form G row groups, each
 // thread holding kBlkRows / G rows of VW columns (fewer accumulators per thread for larger G, so
 // more CTAs fit an SM), with the register budget of M CTAs per SM; OS parks the C values the alpha
@@ -101,6 +102,12 @@ struct Vec<double, 2, kVec> {
   }
 };
 
+struct UnionArgs {
+  const uint32_t *off;  // [row blocks + 1] entries, multiples of 4; null: the pass keeps its per-row doubles
+  const uint32_t *ket;  // ket | rows of the block that have it << 24
+  const void *val;      // [entries][kBlkRows] values of the pass's type
+};
+
 struct BlockArgs {
   // sigma program of the bra spin (rows of X)
   const uint32_t *s_off, *s_ket;
@@ -129,6 +136,7 @@ struct BlockArgs {
   const uint32_t *bs_off, *bs_ket;
   const int32_t *bs_pair;
   const double *eri;
+  UnionArgs u;           // doubles of each row block by distinct ket (dense tables), see sigma_union.cuh
 };
 
 // One kernel, two passes.  A CTA owns kBlkRows consecutive bra strings (rows of X) and a slab of
@@ -835,6 +843,8 @@ __global__ void __launch_bounds__(kBlkThreads, M)
   }
 }
 
+#include "sigma_union.cuh"
+
 }  // namespace
 
 int reorder_sign_apply_f64(sbd_tpb_handle *h, const double *x, double *y) {
@@ -893,13 +903,33 @@ int launch_pass_cm(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T
   return SBD_TPB_OK;
 }
 
+// sigma_union_kernel launch.  Two columns per thread give every SM four CTAs on every problem that gets
+// here (8,192 determinants per SM); FP32 takes four where that still does.
+template <typename T, bool kAlpha, bool kSym>
+int launch_union(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T *XT) {
+  const size_t nrb = (ba.nrows + kBlkRows - 1) / kBlkRows;
+  const size_t smem = ((ba.max_s * 8 + 15) & ~(size_t)15) + (size_t)ba.max_s * 8;
+  auto go = [&](auto kern, size_t cols) -> int {
+    const size_t blocks = nrb * ((ba.ncols + cols - 1) / cols);
+    if (blocks > 0x7fffffffull) return fail(SBD_TPB_ERR_INVALID, "sigma: grid too large");
+    TPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<(unsigned)blocks, kUnionThreads, smem, h->stream>>>(ba, ba.u, X, out, XT);
+    TPB_LAUNCHED(h);
+    return SBD_TPB_OK;
+  };
+  if constexpr (sizeof(T) == 8) return go(sigma_union_kernel<T, kAlpha, kSym, 2, 4>, kUnionThreads * 2);
+  else if (nrb * ((ba.ncols + kUnionThreads * 4 - 1) / (kUnionThreads * 4)) >= 4 * (size_t)h->num_sms)
+    return go(sigma_union_kernel<T, kAlpha, kSym, 4, 4>, kUnionThreads * 4);
+  else return go(sigma_union_kernel<T, kAlpha, kSym, 2, 5>, kUnionThreads * 2);
+}
+
 // Small problems (fewer than 8,192 determinants per SM): the usual tiles (8 rows x 512 FP32 / 256 FP64
 // columns, 4 rows a thread) do not fill the GPU and each thread's chain of gathers is the time.  One
 // row per thread then: an eighth of the columns per CTA, a quarter of the chain.  Same bits.  ms per pass,
 // usual -> one row: 8-orbital full CI FP64 0.028 -> 0.015; 12-orbital 0.196 -> 0.155, FP32 0.130 -> 0.106;
 // 24 orbitals, 1,001 strings FP32 0.046 -> 0.030, 401 dense strings FP64 0.194 -> 0.067; 18 orbitals, 642
-// strings FP64 0.301 -> 0.104.  Above the line it wins less or loses: 18 orbitals, 1,387 strings FP64
-// 0.86 -> 0.81, 24 orbitals, 4,000 strings 0.53 -> 0.67.
+// strings FP64 0.301 -> 0.104 (the union passes 0.186).  Above the line it loses: 18 orbitals, 1,387
+// strings FP64 0.81 against the union passes' 0.49, 24 orbitals, 4,000 strings 0.67 against 0.53.
 inline bool small_problem(const sbd_tpb_handle *h, size_t nrows, size_t ncols) {
   return nrows * ncols < 8192 * (size_t)h->num_sms;
 }
@@ -919,6 +949,7 @@ int launch_block(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T *
   constexpr int VW = 16 / sizeof(T);
   if (!ba.do_ab && small_problem(h, ba.nrows, ba.ncols))
     return launch_block_cfg<T, kAlpha, 8, 8>(h, ba, X, out, XT);
+  if (ba.u.off && !ba.do_ab) return launch_union<T, kAlpha, false>(h, ba, X, out, XT);
   const bool rows16 = (ba.ncols % VW) == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0 && (!XT || reinterpret_cast<uintptr_t>(XT) % 16 == 0);
   if (rows16 && !ba.do_ab) {
@@ -971,11 +1002,139 @@ int launch_sym_cm(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out) {
 template <typename T>
 int launch_block_sym(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out) {
   if (small_problem(h, ba.nrows, ba.ncols)) return launch_block_cfg<T, true, 8, 8, false, true>(h, ba, X, out, nullptr);
+  if (ba.u.off) return launch_union<T, true, true>(h, ba, X, out, nullptr);
   const bool rows16 = (ba.ncols % (16 / sizeof(T))) == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
                       reinterpret_cast<uintptr_t>(out) % 16 == 0;
   if (!rows16) return launch_block_cfg<T, true, 2, 8, false, true>(h, ba, X, out, nullptr);
   if constexpr (sizeof(T) == 4) return launch_sym_cm<T, 4, 10, 2>(h, ba, X, out);
   else return launch_sym_cm<T, 2, 8, 2>(h, ba, X, out);
+}
+
+// The distinct kets of each row block of a doubles table: how many (rounded up to a multiple of 4), and
+// then the list itself, ascending, with the rows that have each ket and their values (zero elsewhere).
+// One CTA per row block; mask holds a byte per ket, pos its place in the list.
+__global__ void __launch_bounds__(256)
+    union_count_kernel(const uint32_t *__restrict__ off, const uint32_t *__restrict__ ket, uint32_t n,
+                       uint32_t *__restrict__ cnt) {
+  extern __shared__ uint32_t mask[];
+  __shared__ uint32_t total;
+  const uint32_t r0 = blockIdx.x * kBlkRows, words = (n + 3) / 4;
+  if (threadIdx.x == 0) total = 0;
+  for (uint32_t w = threadIdx.x; w < words; w += 256) mask[w] = 0;
+  __syncthreads();
+  for (uint32_t r = 0; r < kBlkRows && r0 + r < n; r++)
+    for (uint32_t e = off[r0 + r] + threadIdx.x; e < off[r0 + r + 1]; e += 256)
+      atomicOr(&mask[ket[e] / 4], 1u << (8 * (ket[e] % 4) + r));
+  __syncthreads();
+  uint32_t c = 0;
+  for (uint32_t w = threadIdx.x; w < words; w += 256)
+    for (int k = 0; k < 4; k++) c += (mask[w] >> (8 * k) & 0xff) != 0;
+  atomicAdd(&total, c);
+  __syncthreads();
+  if (threadIdx.x == 0) cnt[blockIdx.x] = (total + 3) & ~3u;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+    union_fill_kernel(const uint32_t *__restrict__ off, const uint32_t *__restrict__ ket, const T *__restrict__ val,
+                      uint32_t n, const uint32_t *__restrict__ uoff, uint32_t *__restrict__ uket, T *__restrict__ uval) {
+  extern __shared__ uint32_t mask[];
+  const uint32_t r0 = blockIdx.x * kBlkRows, words = (n + 3) / 4;
+  uint32_t *pos = mask + words;
+  __shared__ uint32_t warp_sum[8];
+  __shared__ uint32_t carry;
+  const uint32_t u0 = uoff[blockIdx.x], u1 = uoff[blockIdx.x + 1];
+  if (threadIdx.x == 0) carry = 0;
+  for (uint32_t w = threadIdx.x; w < words; w += 256) mask[w] = 0;
+  for (uint32_t e = u0 + threadIdx.x; e < u1; e += 256) uket[e] = 0;
+  for (size_t e = (size_t)u0 * kBlkRows + threadIdx.x; e < (size_t)u1 * kBlkRows; e += 256) uval[e] = T(0);
+  __syncthreads();
+  for (uint32_t r = 0; r < kBlkRows && r0 + r < n; r++)
+    for (uint32_t e = off[r0 + r] + threadIdx.x; e < off[r0 + r + 1]; e += 256)
+      atomicOr(&mask[ket[e] / 4], 1u << (8 * (ket[e] % 4) + r));
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (uint32_t base = 0; base < n; base += 256) {
+    const uint32_t k = base + threadIdx.x;
+    const uint32_t m = k < n ? mask[k / 4] >> (8 * (k % 4)) & 0xff : 0;
+    const uint32_t bal = __ballot_sync(0xffffffffu, m != 0);
+    if (lane == 0) warp_sum[wid] = __popc(bal);
+    __syncthreads();
+    uint32_t p = carry + __popc(bal & ((1u << lane) - 1));
+    for (int w = 0; w < wid; w++) p += warp_sum[w];
+    if (m) {
+      pos[k] = p;
+      uket[u0 + p] = k | m << 24;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 0; w < 8; w++) carry += warp_sum[w];
+    __syncthreads();
+  }
+  for (uint32_t r = 0; r < kBlkRows && r0 + r < n; r++)
+    for (uint32_t e = off[r0 + r] + threadIdx.x; e < off[r0 + r + 1]; e += 256)
+      uval[((size_t)u0 + pos[ket[e]]) * kBlkRows + r] = val[e];
+}
+
+// The union list of a sigma program (n strings), built on first use per problem and type; left out
+// (u_off null) where rows share too few kets, its singles have no Coulomb table, or it would take
+// more than an eighth of the free memory.
+template <typename T>
+int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, UnionArgs *u) {
+  *u = UnionArgs();
+  if (!p.u_tried) {
+    p.u_tried = true;
+    const size_t smem = (n + 3) / 4 * 4 + n * 4, nblk = (n + kBlkRows - 1) / kBlkRows;
+    if (p.d->nnz == 0 || n >= (1u << 24) || smem + 1024 > h->smem_optin || (p.s->nnz && !p.jtab)) return SBD_TPB_OK;
+    uint32_t *d_cnt = nullptr;
+    std::vector<uint32_t> off(nblk + 1, 0);
+    TPB_CUDA(cudaMalloc(&d_cnt, sizeof(uint32_t) * nblk));
+    TPB_CUDA(cudaFuncSetAttribute(union_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    union_count_kernel<<<(unsigned)nblk, 256, smem, h->stream>>>(p.d->off, p.d->ket, (uint32_t)n, d_cnt);
+    h->launches++;
+    const cudaError_t e1 = cudaGetLastError();
+    const cudaError_t e2 = e1 != cudaSuccess ? e1
+                                             : cudaMemcpyAsync(off.data() + 1, d_cnt, sizeof(uint32_t) * nblk,
+                                                               cudaMemcpyDeviceToHost, h->stream);
+    const cudaError_t e3 = e2 != cudaSuccess ? e2 : cudaStreamSynchronize(h->stream);
+    cudaFree(d_cnt);
+    if (e3 != cudaSuccess) return fail(SBD_TPB_ERR_CUDA, std::string("union list: ") + cudaGetErrorString(e3));
+    size_t total = 0;
+    for (size_t b = 0; b < nblk; b++) {
+      total += off[b + 1];
+      if (total > 0xfffffff0ull) return SBD_TPB_OK;
+      off[b + 1] = (uint32_t)total;
+    }
+    if ((double)p.d->nnz < kUnionReuse * (double)total) return SBD_TPB_OK;
+    TPB_CUDA(cudaMalloc(&p.u_off, sizeof(uint32_t) * (nblk + 1)));
+    TPB_CUDA(cudaMemcpy(p.u_off, off.data(), sizeof(uint32_t) * (nblk + 1), cudaMemcpyHostToDevice));
+    p.u_total = total;
+  }
+  if (!p.u_off) return SBD_TPB_OK;
+  T **val = reinterpret_cast<T **>(sizeof(T) == 8 ? (void **)&p.u_val : (void **)&p.u_valf);
+  if (!*val) {
+    const size_t bytes = sizeof(T) * kBlkRows * p.u_total, smem = (n + 3) / 4 * 4 + n * 4;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 8) {
+      cudaGetLastError();
+      return SBD_TPB_OK;
+    }
+    if (!p.u_ket) TPB_CUDA(cudaMalloc(&p.u_ket, sizeof(uint32_t) * p.u_total));
+    if (cudaMalloc(val, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      *val = nullptr;
+      return SBD_TPB_OK;
+    }
+    const T *src = reinterpret_cast<const T *>(sizeof(T) == 8 ? (const void *)p.d_val : (const void *)p.d_valf);
+    TPB_CUDA(cudaFuncSetAttribute(union_fill_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    union_fill_kernel<T><<<(unsigned)((n + kBlkRows - 1) / kBlkRows), 256, smem, h->stream>>>(
+        p.d->off, p.d->ket, src, (uint32_t)n, p.u_off, p.u_ket, *val);
+    TPB_LAUNCHED(h);
+  }
+  u->off = p.u_off;
+  u->ket = p.u_ket;
+  u->val = *val;
+  return SBD_TPB_OK;
 }
 
 // Most entries of any kBlkRows-row block of a CSR table of n rows (shared-memory staging size).
@@ -1173,8 +1332,14 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
   // per-pair Coulomb sums of the singles over the other spin's strings (built once per problem)
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   TPB_CHECK(build_coulomb_table(h, h->pb, h->d_astr, na));
+  UnionArgs ua, ub;
+  if (!small_problem(h, na, nb)) {
+    TPB_CHECK(build_union<T>(h, h->pa, na, &ua));
+    TPB_CHECK(build_union<T>(h, h->pb, nb, &ub));
+  }
 
   BlockArgs ba{};
+  ba.u = ua;
   ba.s_off = h->ta_s.off;
   ba.s_ket = h->ta_s.ket;
   ba.s_val = h->pa.s_val;
@@ -1207,6 +1372,7 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
   TPB_CUDA(cudaEventRecord(h->ev_k[0], h->stream));
 
   BlockArgs bb{};
+  bb.u = ub;
   bb.s_off = h->tb_s.off;
   bb.s_ket = h->tb_s.ket;
   bb.s_val = h->pb.s_val;
@@ -1260,7 +1426,10 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
   const bool rows_ab = h->abr.ready && !dense_ab;
   TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab));
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
+  UnionArgs ua;
+  if (!small_problem(h, na, nb)) TPB_CHECK(build_union<T>(h, h->pa, na, &ua));
   BlockArgs ba{};
+  ba.u = ua;
   ba.s_off = h->ta_s.off;
   ba.s_ket = h->ta_s.ket;
   ba.s_val = h->pa.s_val;

@@ -102,6 +102,12 @@ struct SigmaProg {
   int32_t *pmap = nullptr;
   uint32_t npair = 0;
   bool jtab_tried = false;  // built, or found too large, once per program
+  // doubles of each 8-row block by distinct ket (build_union, sigma.cu): dense tables only
+  uint32_t *u_off = nullptr, *u_ket = nullptr;
+  double *u_val = nullptr;
+  float *u_valf = nullptr;
+  size_t u_total = 0;
+  bool u_tried = false;
 };
 
 // Dense-path data for the alpha-beta term as gather -> (pq|rs) contraction -> scatter.

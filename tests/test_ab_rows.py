@@ -1,5 +1,7 @@
-"""The alpha-beta term of densely connected string sets (csrc/ab_rows.cu: one product per alpha row and
-a gather over the beta singles) against the oracle, at the sizes where its tiling can go wrong.
+"""Sigma on densely connected string sets -- the alpha-beta term (csrc/ab_rows.cu: one product per alpha
+row and a gather over the beta singles) and the same-spin passes (csrc/sigma_union.cuh from 8,192
+determinants per SM, one row per thread below) -- against the oracle, at the sizes where their tiling can
+go wrong.
 
 Sets: n strings of lowest orbital-index sum with noise, so that they hold tens of singles each.  Column
 steps are 32 wide, rows of the product come in blocks of 8 (one pass up to 24 blocks), singles in groups
@@ -30,6 +32,8 @@ CASES = {
     "two_groups": (18, (7, 600), (7, 600)),    # up to 77 singles in a row: two groups of at most 64
     "two_passes": (24, (5, 401), (4, 333)),    # up to 276 pairs: two passes over the rows of the product
     "one_row": (10, (5, 2), (5, 252)),         # rows with a single single
+    "union": (18, (7, 1101), (7, 1103)),       # just above the line of the union passes: narrow FP32 tiles
+    "many_blocks": (18, (7, 1400), (7, 2101)),  # the widest thread tiles of the same-spin passes, odd rows
     "wide": (18, (7, 24), (7, 15001)),         # a sigma row longer than shared memory holds in FP64
 }
 
