@@ -184,10 +184,11 @@ int ab_dense_setup(sbd_tpb_handle *h, int enable) {
   TPB_CUDA(cudaMalloc(&ab.b_label, sizeof(int32_t) * blab.size()));
   TPB_CUDA(cudaMalloc(&ab.V, sizeof(double) * V.size()));
   TPB_CUDA(cudaMalloc(&ab.Vf, sizeof(float) * Vf.size()));
-  TPB_CUDA(cudaMemcpy(ab.a_label, alab.data(), sizeof(int32_t) * alab.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(ab.b_label, blab.data(), sizeof(int32_t) * blab.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(ab.V, V.data(), sizeof(double) * V.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(ab.Vf, Vf.data(), sizeof(float) * Vf.size(), cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, ab.a_label, alab.data(), sizeof(int32_t) * alab.size()));
+  TPB_CUDA(h2d(h, ab.b_label, blab.data(), sizeof(int32_t) * blab.size()));
+  TPB_CUDA(h2d(h, ab.V, V.data(), sizeof(double) * V.size()));
+  TPB_CUDA(h2d(h, ab.Vf, Vf.data(), sizeof(float) * Vf.size()));
+  TPB_CUDA(cudaStreamSynchronize(h->stream));
   TPB_CHECK(ab_tc_setup(h));
   ab.enabled = true;
   (void)n;

@@ -388,9 +388,9 @@ int launch_rows(sbd_tpb_handle *h, RowArgs a, const T *C, T *sigma) {
 }
 
 template <typename T>
-int upload(T **dst, const std::vector<T> &src) {
+int upload(sbd_tpb_handle *h, T **dst, const std::vector<T> &src) {
   TPB_CUDA(cudaMalloc(dst, sizeof(T) * std::max<size_t>(1, src.size())));
-  if (!src.empty()) TPB_CUDA(cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, *dst, src.data(), sizeof(T) * src.size()));
   return SBD_TPB_OK;
 }
 
@@ -528,12 +528,13 @@ int ab_rows_prepare(sbd_tpb_handle *h) {
   hdr[ncell] = make_uint4((uint32_t)prog.size(), 0, 0, 0);
   r.prog_cap = (uint32_t)cap;
   if (rows_smem(r, sizeof(double), nb, false, 2) > h->smem_optin) return SBD_TPB_OK;
-  TPB_CHECK(upload(&r.rows, rows));
-  TPB_CHECK(upload(&r.ent, ent));
-  TPB_CHECK(upload(&r.pair_m, pair_m));
-  TPB_CHECK(upload(&r.m_pair, m_pair));
-  TPB_CHECK(upload(&r.hdr, hdr));
-  TPB_CHECK(upload(&r.prog, prog));
+  TPB_CHECK(upload(h, &r.rows, rows));
+  TPB_CHECK(upload(h, &r.ent, ent));
+  TPB_CHECK(upload(h, &r.pair_m, pair_m));
+  TPB_CHECK(upload(h, &r.m_pair, m_pair));
+  TPB_CHECK(upload(h, &r.hdr, hdr));
+  TPB_CHECK(upload(h, &r.prog, prog));
+  TPB_CUDA(cudaStreamSynchronize(h->stream));
   TPB_CUDA(cudaHostAlloc(&r.err, sizeof(int), cudaHostAllocMapped));
   *r.err = 0;
   r.ready = true;

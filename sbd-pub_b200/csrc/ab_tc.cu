@@ -387,10 +387,11 @@ int ab_tc_setup(sbd_tpb_handle *h) {
     }
   TPB_CUDA(cudaMalloc(&ab.Vhi, sizeof(uint16_t) * hi.size()));
   TPB_CUDA(cudaMalloc(&ab.Vlo, sizeof(uint16_t) * lo.size()));
-  TPB_CUDA(cudaMemcpy(ab.Vhi, hi.data(), sizeof(uint16_t) * hi.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(ab.Vlo, lo.data(), sizeof(uint16_t) * lo.size(), cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, ab.Vhi, hi.data(), sizeof(uint16_t) * hi.size()));
+  TPB_CUDA(h2d(h, ab.Vlo, lo.data(), sizeof(uint16_t) * lo.size()));
   if (!ab.err) TPB_CUDA(cudaMalloc(&ab.err, sizeof(int)));
-  TPB_CUDA(cudaMemset(ab.err, 0, sizeof(int)));
+  TPB_CUDA(cudaMemsetAsync(ab.err, 0, sizeof(int), h->stream));
+  TPB_CUDA(cudaStreamSynchronize(h->stream));
   TPB_CUDA(cudaFuncSetAttribute(ab_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // fused gather + contraction: two accumulators of up to 256 columns, V resident, one or two A stages
   ab.tc_fused_stages = 0;
@@ -461,7 +462,7 @@ int ab_tc_check(sbd_tpb_handle *h) {
   int e = 0;
   TPB_CUDA(cudaMemcpy(&e, h->ab.err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e) {
-    cudaMemset(h->ab.err, 0, sizeof(int));
+    cudaMemsetAsync(h->ab.err, 0, sizeof(int), h->stream);
     return fail(SBD_TPB_ERR_CUDA, "alpha-beta tensor-core kernel: bounded wait expired (code " +
                                       std::to_string(e) + ")");
   }

@@ -25,6 +25,10 @@ int fail(int code, const std::string &msg) {
   return code;
 }
 
+cudaError_t h2d(sbd_tpb_handle *h, void *dst, const void *src, size_t bytes) {
+  return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream) : cudaSuccess;
+}
+
 }  // namespace sbdtpb
 
 using namespace sbdtpb;

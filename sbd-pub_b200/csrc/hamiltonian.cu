@@ -198,8 +198,8 @@ int build_coulomb_table(sbd_tpb_handle *h, SigmaProg &p, const uint64_t *col_str
   int32_t *d_pairs = nullptr;
   TPB_CUDA(cudaMalloc(&p.pmap, sizeof(int32_t) * L2));
   TPB_CUDA(cudaMalloc(&d_pairs, sizeof(int32_t) * pairs.size()));
-  TPB_CUDA(cudaMemcpy(p.pmap, pmap.data(), sizeof(int32_t) * L2, cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(d_pairs, pairs.data(), sizeof(int32_t) * pairs.size(), cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, p.pmap, pmap.data(), sizeof(int32_t) * L2));
+  TPB_CUDA(h2d(h, d_pairs, pairs.data(), sizeof(int32_t) * pairs.size()));
   p.npair = (uint32_t)pairs.size();
   const size_t tot = pairs.size() * ncols;
   coulomb_table_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, h->stream>>>(col_str, ncols, d_pairs, p.npair,
@@ -294,11 +294,12 @@ int upload_hamiltonian(sbd_tpb_handle *h) {
   TPB_CUDA(cudaMalloc(&h->d_eri, sizeof(double) * eri.size()));
   TPB_CUDA(cudaMalloc(&h->d_vd, sizeof(double) * vd.size()));
   TPB_CUDA(cudaMalloc(&h->d_J, sizeof(double) * (J.size() + L2)));
-  TPB_CUDA(cudaMemcpy(h->d_eri, eri.data(), sizeof(double) * eri.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_vd, vd.data(), sizeof(double) * vd.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_J, J.data(), sizeof(double) * J.size(), cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, h->d_eri, eri.data(), sizeof(double) * eri.size()));
+  TPB_CUDA(h2d(h, h->d_vd, vd.data(), sizeof(double) * vd.size()));
+  TPB_CUDA(h2d(h, h->d_J, J.data(), sizeof(double) * J.size()));
   // the one-electron matrix rides behind J
-  TPB_CUDA(cudaMemcpy(h->d_J + L2, h->h1.data(), sizeof(double) * L2, cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, h->d_J + L2, h->h1.data(), sizeof(double) * L2));
+  TPB_CUDA(cudaStreamSynchronize(h->stream));
   return SBD_TPB_OK;
 }
 
@@ -342,12 +343,13 @@ int build_string_data(sbd_tpb_handle *h) {
   TPB_CUDA(cudaMalloc(&h->d_Ea, sizeof(double) * na));
   TPB_CUDA(cudaMalloc(&h->d_Eb, sizeof(double) * nb));
   TPB_CUDA(cudaMalloc(&h->d_uJ, sizeof(double) * na * L));
-  TPB_CUDA(cudaMemcpy(h->d_astr, h->astr.data(), sizeof(uint64_t) * na, cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_bstr, h->bstr.data(), sizeof(uint64_t) * nb, cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_apar, apar.data(), sizeof(uint64_t) * na, cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_Ea, Ea.data(), sizeof(double) * na, cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_Eb, Eb.data(), sizeof(double) * nb, cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_uJ, uJ.data(), sizeof(double) * na * L, cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, h->d_astr, h->astr.data(), sizeof(uint64_t) * na));
+  TPB_CUDA(h2d(h, h->d_bstr, h->bstr.data(), sizeof(uint64_t) * nb));
+  TPB_CUDA(h2d(h, h->d_apar, apar.data(), sizeof(uint64_t) * na));
+  TPB_CUDA(h2d(h, h->d_Ea, Ea.data(), sizeof(double) * na));
+  TPB_CUDA(h2d(h, h->d_Eb, Eb.data(), sizeof(double) * nb));
+  TPB_CUDA(h2d(h, h->d_uJ, uJ.data(), sizeof(double) * na * L));
+  TPB_CUDA(cudaStreamSynchronize(h->stream));
   return SBD_TPB_OK;
 }
 

@@ -986,10 +986,11 @@ int ensure_occ_windows(sbd_tpb_handle *h) {
   TPB_CUDA(cudaMalloc(&h->d_occw_b, sizeof(uint32_t) * std::max<size_t>(1, b.size())));
   TPB_CUDA(cudaMalloc(&h->d_kx_a, sizeof(double) * std::max<size_t>(1, ka.size())));
   TPB_CUDA(cudaMalloc(&h->d_kx_b, sizeof(double) * std::max<size_t>(1, kb.size())));
-  TPB_CUDA(cudaMemcpy(h->d_occw_a, a.data(), sizeof(uint32_t) * a.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_occw_b, b.data(), sizeof(uint32_t) * b.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_kx_a, ka.data(), sizeof(double) * ka.size(), cudaMemcpyHostToDevice));
-  TPB_CUDA(cudaMemcpy(h->d_kx_b, kb.data(), sizeof(double) * kb.size(), cudaMemcpyHostToDevice));
+  TPB_CUDA(h2d(h, h->d_occw_a, a.data(), sizeof(uint32_t) * a.size()));
+  TPB_CUDA(h2d(h, h->d_occw_b, b.data(), sizeof(uint32_t) * b.size()));
+  TPB_CUDA(h2d(h, h->d_kx_a, ka.data(), sizeof(double) * ka.size()));
+  TPB_CUDA(h2d(h, h->d_kx_b, kb.data(), sizeof(double) * kb.size()));
+  TPB_CUDA(cudaStreamSynchronize(h->stream));
   return SBD_TPB_OK;
 }
 
@@ -1171,7 +1172,8 @@ int precond_apply(sbd_tpb_handle *h, sbd_tpb_precond *p, T *t, double e0, double
   TPB_CUDA(cudaMemcpyAsync(&e, p->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   TPB_CUDA(cudaStreamSynchronize(h->stream));
   if (e) {
-    cudaMemset(p->err, 0, sizeof(int));
+    cudaMemsetAsync(p->err, 0, sizeof(int), h->stream);
+    cudaStreamSynchronize(h->stream);  // before the training kernels' next use of it on p->stream
     return fail(SBD_TPB_ERR_CUDA, "learned preconditioner: tensor-core wait expired (code " + std::to_string(e) + ")");
   }
   return SBD_TPB_OK;
@@ -1263,11 +1265,11 @@ extern "C" int sbd_tpb_precond_create(int device, uint64_t seed, sbd_tpb_precond
   for (int o = 0; o < H; o++)
     for (int k = 0; k < 2 + 2 * kMlpWin; k++) P[oW1 + (size_t)o * F + k] = n1(g);
   for (size_t i = 0; i < (size_t)H * H; i++) P[oW2 + i] = n2(g);
-  cudaMemcpy(p->P, P.data(), kParams * 4, cudaMemcpyHostToDevice);
-  cudaMemset(p->m, 0, kParams * 4);
-  cudaMemset(p->v, 0, kParams * 4);
-  cudaMemset(p->G, 0, kParams * 4);
-  cudaMemset(p->err, 0, sizeof(int));
+  cudaMemcpyAsync(p->P, P.data(), kParams * 4, cudaMemcpyHostToDevice, p->stream);
+  cudaMemsetAsync(p->m, 0, kParams * 4, p->stream);
+  cudaMemsetAsync(p->v, 0, kParams * 4, p->stream);
+  cudaMemsetAsync(p->G, 0, kParams * 4, p->stream);
+  cudaMemsetAsync(p->err, 0, sizeof(int), p->stream);
   if (pack_weights(p) != SBD_TPB_OK || cudaStreamSynchronize(p->stream) != cudaSuccess) {
     delete p;
     return fail(SBD_TPB_ERR_CUDA, "precond: init");

@@ -519,9 +519,10 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
       TPB_CUDA(cudaMalloc(&lb.seg, sizeof(uint32_t) * seg.size()));
       TPB_CUDA(cudaMalloc(&lb.ord, sizeof(int32_t) * std::max<size_t>(1, w)));
       TPB_CUDA(cudaMalloc(&lb.bra, sizeof(uint64_t) * std::max<size_t>(1, w)));
-      TPB_CUDA(cudaMemcpy(lb.seg, seg.data(), sizeof(uint32_t) * seg.size(), cudaMemcpyHostToDevice));
-      TPB_CUDA(cudaMemcpy(lb.ord, ord.data(), sizeof(int32_t) * w, cudaMemcpyHostToDevice));
-      TPB_CUDA(cudaMemcpy(lb.bra, bra.data(), sizeof(uint64_t) * w, cudaMemcpyHostToDevice));
+      TPB_CUDA(h2d(h, lb.seg, seg.data(), sizeof(uint32_t) * seg.size()));
+      TPB_CUDA(h2d(h, lb.ord, ord.data(), sizeof(int32_t) * w));
+      TPB_CUDA(h2d(h, lb.bra, bra.data(), sizeof(uint64_t) * w));
+      TPB_CUDA(cudaStreamSynchronize(h->stream));
       return SBD_TPB_OK;
     };
     Labels la, lbeta;
@@ -633,9 +634,9 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
       TPB_CUDA(cudaMalloc(&d_bbra, sizeof(uint32_t) * bbra.size()));
       TPB_CUDA(cudaMalloc(&d_blab, sizeof(int32_t) * blab.size()));
       TPB_CUDA(cudaMalloc(&d_X, sizeof(double) * h->ta_s.nnz * L2));
-      TPB_CUDA(cudaMemcpy(d_abra, abra.data(), sizeof(uint32_t) * abra.size(), cudaMemcpyHostToDevice));
-      TPB_CUDA(cudaMemcpy(d_bbra, bbra.data(), sizeof(uint32_t) * bbra.size(), cudaMemcpyHostToDevice));
-      TPB_CUDA(cudaMemcpy(d_blab, blab.data(), sizeof(int32_t) * blab.size(), cudaMemcpyHostToDevice));
+      TPB_CUDA(h2d(h, d_abra, abra.data(), sizeof(uint32_t) * abra.size()));
+      TPB_CUDA(h2d(h, d_bbra, bbra.data(), sizeof(uint32_t) * bbra.size()));
+      TPB_CUDA(h2d(h, d_blab, blab.data(), sizeof(int32_t) * blab.size()));
       rdm_mixed_kernel<<<(unsigned)h->ta_s.nnz, kRdmThreads, sizeof(double) * L2, h->stream>>>(
           W, nb, d_abra, h->ta_s.ket, d_bbra, h->tb_s.ket, d_blab, (uint32_t)h->tb_s.nnz, L2, d_X);
       TPB_LAUNCHED(h);

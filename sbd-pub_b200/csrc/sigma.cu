@@ -1110,7 +1110,8 @@ int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, UnionArgs *u) {
     }
     if ((double)p.d->nnz < kUnionReuse * (double)total) return SBD_TPB_OK;
     TPB_CUDA(cudaMalloc(&p.u_off, sizeof(uint32_t) * (nblk + 1)));
-    TPB_CUDA(cudaMemcpy(p.u_off, off.data(), sizeof(uint32_t) * (nblk + 1), cudaMemcpyHostToDevice));
+    TPB_CUDA(h2d(h, p.u_off, off.data(), sizeof(uint32_t) * (nblk + 1)));
+    TPB_CUDA(cudaStreamSynchronize(h->stream));
     p.u_total = total;
   }
   if (!p.u_off) return SBD_TPB_OK;
@@ -1251,12 +1252,13 @@ int prepare_sigma_meta(sbd_tpb_handle *h, bool want_ab_lists) {
     TPB_CUDA(cudaMalloc(&h->d_ab_colp, sizeof(uint2) * colp.size()));
     TPB_CUDA(cudaMalloc(&h->d_ab_bsp, sizeof(uint2) * bsp.size()));
     TPB_CUDA(cudaMalloc(&h->d_ab_kets, sizeof(uint32_t) * kets.size()));
-    TPB_CUDA(cudaMemcpy(h->d_ab_kets, kets.data(), sizeof(uint32_t) * kets.size(), cudaMemcpyHostToDevice));
+    TPB_CUDA(h2d(h, h->d_ab_kets, kets.data(), sizeof(uint32_t) * kets.size()));
     h->ab_nkets = nnz ? (uint32_t)kets.size() : 0;
     if (!rows.empty())
-      TPB_CUDA(cudaMemcpy(h->d_ab_rows, rows.data(), sizeof(uint32_t) * rows.size(), cudaMemcpyHostToDevice));
-    TPB_CUDA(cudaMemcpy(h->d_ab_colp, colp.data(), sizeof(uint2) * colp.size(), cudaMemcpyHostToDevice));
-    TPB_CUDA(cudaMemcpy(h->d_ab_bsp, bsp.data(), sizeof(uint2) * bsp.size(), cudaMemcpyHostToDevice));
+      TPB_CUDA(h2d(h, h->d_ab_rows, rows.data(), sizeof(uint32_t) * rows.size()));
+    TPB_CUDA(h2d(h, h->d_ab_colp, colp.data(), sizeof(uint2) * colp.size()));
+    TPB_CUDA(h2d(h, h->d_ab_bsp, bsp.data(), sizeof(uint2) * bsp.size()));
+    TPB_CUDA(cudaStreamSynchronize(h->stream));
     h->ab_nrows = (uint32_t)rows.size();
     h->ab_ncols = (uint32_t)ncs;
     h->ab_max_k = kmax;

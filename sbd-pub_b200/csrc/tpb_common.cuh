@@ -51,6 +51,11 @@ int fail(int code, const std::string &msg);
     if (rc_ != SBD_TPB_OK) return rc_; \
   } while (0)
 
+// Host -> device copy ordered before what h->stream runs next.  (cudaMemcpy runs on the legacy stream and may
+// return while a pageable source is only staged; the handle's stream is non-blocking and would not wait for
+// it.)  Functions whose sources are locals synchronise the stream once after their last copy.
+cudaError_t h2d(sbd_tpb_handle *h, void *dst, const void *src, size_t bytes);
+
 // ---- device bit helpers ---------------------------------------------------------------------
 __host__ __device__ __forceinline__ uint64_t open_mask(int lo, int hi) {
   // bits strictly between lo and hi (0 <= lo < hi <= 63)

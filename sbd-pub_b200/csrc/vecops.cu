@@ -1170,7 +1170,7 @@ constexpr int kRrDoubles = kMaxSub * kMaxSub + 2 * kMaxSub;
 static int ensure_scalars(sbd_tpb_handle *h) {
   if (h->d_scal) return SBD_TPB_OK;
   TPB_CUDA(cudaMalloc(&h->d_scal, sizeof(double) * (kScalarSlots + kRrDoubles)));
-  TPB_CUDA(cudaMemset(h->d_scal, 0, sizeof(double) * (kScalarSlots + kRrDoubles)));
+  TPB_CUDA(cudaMemsetAsync(h->d_scal, 0, sizeof(double) * (kScalarSlots + kRrDoubles), h->stream));
   TPB_CUDA(cudaMallocHost(&h->h_scal, sizeof(double) * kScalarSlots));
   return SBD_TPB_OK;
 }
