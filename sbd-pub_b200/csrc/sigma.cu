@@ -26,10 +26,6 @@ namespace {
 
 constexpr int kBlkRows = 8;  // bra rows per CTA
 constexpr int kBlkThreads = 128;
-// Doubles per distinct ket of a row block from which the union passes run: molecular sets have 2.0 to 2.6
-// (2.1 at 18 orbitals, 4,041 strings: 11.9 -> 4.3 ms a pass), sampled selected sets 1.12 to 1.2, where nothing is
-// shared and the wider per-row tiles keep their lead; no set in use lies between.
-constexpr double kUnionReuse = 1.5;
 // Thread mapping of a CTA per element type and pass: the 128 threads form G row groups, each
 // thread holding kBlkRows / G rows of VW columns (fewer accumulators per thread for larger G, so
 // more CTAs fit an SM), with the register budget of M CTAs per SM; OS parks the C values the alpha
@@ -864,6 +860,13 @@ int reorder_sign_apply_f32(sbd_tpb_handle *h, const float *x, float *y) {
   return SBD_TPB_OK;
 }
 
+// Whether 16-byte column accesses may be used: every row of each buffer starts 16-byte aligned.
+template <typename T>
+inline bool rows_aligned(size_t ncols, const T *a, const T *b, const T *c = nullptr) {
+  return ncols % (16 / sizeof(T)) == 0 &&
+         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) % 16) == 0;
+}
+
 template <typename T, bool kAlpha, int G, int M, bool OS = false, bool kSym = false>
 int launch_block_cfg(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T *XT) {
   constexpr int VW = 16 / sizeof(T);
@@ -876,9 +879,7 @@ int launch_block_cfg(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out,
                       (OS ? (size_t)(kBlkRows / G) * VW * kBlkThreads * sizeof(T) + 16 : 0);
   if (smem > h->smem_optin) return fail(SBD_TPB_ERR_INVALID, "sigma: table block exceeds shared memory");
   // 16-byte column accesses need every row of X to start 16-byte aligned
-  const bool vec = (ba.ncols % VW) == 0 && (reinterpret_cast<uintptr_t>(X) % 16) == 0 &&
-                   (reinterpret_cast<uintptr_t>(out) % 16) == 0 &&
-                   (!XT || (reinterpret_cast<uintptr_t>(XT) % 16) == 0);
+  const bool vec = rows_aligned(ba.ncols, X, out, XT);
   auto kern = vec ? sigma_block_kernel<T, kAlpha, true, G, M, OS, kSym>
                   : sigma_block_kernel<T, kAlpha, false, G, M, OS, kSym>;
   TPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -937,6 +938,29 @@ inline bool small_problem(const sbd_tpb_handle *h, size_t nrows, size_t ncols) {
   return nrows * ncols < 8192 * (size_t)h->num_sms;
 }
 
+// Whether the union passes are ahead of the per-row ones, from the doubles per distinct ket of a row
+// block (`reuse`), the largest block's table entries and the kind of column access.  The per-row passes
+// stage a block's whole table, so few of their CTAs fit an SM when it is large; the union passes stage
+// 64 kets at a time whatever its size.  At equal residency a per-row pass takes about 0.42 (FP64) and
+// 0.36 to 0.43 (FP32) of a union pass's time per unit of reuse with 16-byte rows, 0.6 with scalar ones; with
+// 3, 2 and 1 CTAs fitting an SM FP64 takes 0.62, 0.88 and 1.6.  The lines are where the products reach 1.
+// ms of one pass, per row / union (reuse, CTAs that fit): FP64, 16-byte rows: 20 orbitals, 2,000 strings
+// (1.75, 7) 0.40 / 0.47; 22, 6,000 (1.58, 4) 3.7 / 4.6; 26, 16,000 (1.38, 3) 25.2 / 28.3; 20, 6,000 (1.82, 3)
+// 8.6 / 7.7; 24, 16,000 (1.46, 2) 49 / 38; 18 molecular, 4,040 (2.14, 2) 7.7 / 4.3; 26 molecular, 3,900 (2.10, 1)
+// 16.2 / 5.0.  FP32: 20, 6,000 (1.82, 4) 4.7 / 5.6; 22, 16,000 (1.64, 3) sum of both passes 84.5 / 92.9; 18
+// molecular, 4,040 (2.14, 3) 4.2 / 3.1; 18 molecular, 1,388 (2.40, 5) 0.45 / 0.33; 20, 14,000 (1.89, 2) 67.5 / 56.7.
+// Scalar rows, FP64: 22, 4,001 (1.54, 6) 1.44 / 1.61; 22, 6,001 (1.58, 4) 5.3 / 4.7; 24, 8,001 (1.42, 4) sum 12.8 /
+// 11.9; 18 molecular, 4,041 (2.14, 2) 12.1 / 4.3.  FP32: 22, 6,001 (1.58, 6) sum 6.56 / 6.87; 20, 2,001 (1.76, 8)
+// 0.41 / 0.39; 20, 6,001 (1.82, 4) 7.0 / 5.7; 18 molecular, 1,387 (2.40, 5) 0.58 / 0.33.
+template <typename T>
+bool union_ahead(const sbd_tpb_handle *h, double reuse, size_t max_d, size_t max_s, bool rows16) {
+  constexpr int kMost = 5;  // residency beyond which the line stays
+  static constexpr double line[2][2][kMost + 1] = {{{0.0, 1.15, 1.15, 1.15, 1.4, 1.65}, {0.0, 1.15, 1.15, 1.65, 2.1, 2.1}},
+                                                   {{0.0, 1.15, 1.15, 1.15, 1.45, 1.75}, {0.0, 1.5, 1.5, 2.0, 2.35, 2.35}}};
+  const size_t ctas = (h->smem_optin + 1024) / (max_d * (4 + sizeof(T)) + max_s * 16 + 1024);
+  return reuse > 0.0 && reuse >= line[sizeof(T) == 4][rows16][std::min<size_t>(ctas, kMost)];
+}
+
 // Launch shapes of the general passes.  16-byte rows without the alpha-single x beta-single terms
 // take sigma_pass_cm_kernel; from a sweep (CUDA events, ms at 4e8 / 1e8 determinants, row groups /
 // CTAs per SM / column groups, "os": own values parked in shared memory), all giving the same bits:
@@ -949,13 +973,10 @@ inline bool small_problem(const sbd_tpb_handle *h, size_t nrows, size_t ncols) {
 // for C^T parked in shared memory above.
 template <typename T, bool kAlpha>
 int launch_block(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out, T *XT) {
-  constexpr int VW = 16 / sizeof(T);
   if (!ba.do_ab && small_problem(h, ba.nrows, ba.ncols))
     return launch_block_cfg<T, kAlpha, 8, 8>(h, ba, X, out, XT);
   if (ba.u.off && !ba.do_ab) return launch_union<T, kAlpha, false>(h, ba, X, out, XT);
-  const bool rows16 = (ba.ncols % VW) == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
-                      reinterpret_cast<uintptr_t>(out) % 16 == 0 && (!XT || reinterpret_cast<uintptr_t>(XT) % 16 == 0);
-  if (rows16 && !ba.do_ab) {
+  if (rows_aligned(ba.ncols, X, out, XT) && !ba.do_ab) {
     if constexpr (sizeof(T) == 4 && kAlpha) return launch_pass_cm<T, true, 2, 7, 2, true>(h, ba, X, out, XT);
     else if constexpr (sizeof(T) == 4) return launch_pass_cm<T, false, 2, 8, 2>(h, ba, X, out, XT);
     else if constexpr (kAlpha) return launch_pass_cm<T, true, 2, 7, 2>(h, ba, X, out, XT);
@@ -1006,9 +1027,7 @@ template <typename T>
 int launch_block_sym(sbd_tpb_handle *h, const BlockArgs &ba, const T *X, T *out) {
   if (small_problem(h, ba.nrows, ba.ncols)) return launch_block_cfg<T, true, 8, 8, false, true>(h, ba, X, out, nullptr);
   if (ba.u.off) return launch_union<T, true, true>(h, ba, X, out, nullptr);
-  const bool rows16 = (ba.ncols % (16 / sizeof(T))) == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0 &&
-                      reinterpret_cast<uintptr_t>(out) % 16 == 0;
-  if (!rows16) return launch_block_cfg<T, true, 2, 8, false, true>(h, ba, X, out, nullptr);
+  if (!rows_aligned(ba.ncols, X, out)) return launch_block_cfg<T, true, 2, 8, false, true>(h, ba, X, out, nullptr);
   if constexpr (sizeof(T) == 4) return launch_sym_cm<T, 4, 10, 2>(h, ba, X, out);
   else return launch_sym_cm<T, 2, 8, 2>(h, ba, X, out);
 }
@@ -1079,11 +1098,11 @@ __global__ void __launch_bounds__(256)
       uval[((size_t)u0 + pos[ket[e]]) * kBlkRows + r] = val[e];
 }
 
-// The union list of a sigma program (n strings), built on first use per problem and type; left out
-// (u_off null) where rows share too few kets, its singles have no Coulomb table, or it would take
-// more than an eighth of the free memory.
+// The union list of a sigma program (n strings, blk: its entries of h->blk_max), built on first use per
+// problem and type; left out (u->off null) where the per-row passes are ahead, the singles have no
+// Coulomb table, or it would take more than an eighth of the free memory.
 template <typename T>
-int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, UnionArgs *u) {
+int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, int blk, bool rows16, UnionArgs *u) {
   *u = UnionArgs();
   if (!p.u_tried) {
     p.u_tried = true;
@@ -1108,13 +1127,13 @@ int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, UnionArgs *u) {
       if (total > 0xfffffff0ull) return SBD_TPB_OK;
       off[b + 1] = (uint32_t)total;
     }
-    if ((double)p.d->nnz < kUnionReuse * (double)total) return SBD_TPB_OK;
+    p.u_reuse = (double)p.d->nnz / (double)total;
     TPB_CUDA(cudaMalloc(&p.u_off, sizeof(uint32_t) * (nblk + 1)));
     TPB_CUDA(h2d(h, p.u_off, off.data(), sizeof(uint32_t) * (nblk + 1)));
     TPB_CUDA(cudaStreamSynchronize(h->stream));
     p.u_total = total;
   }
-  if (!p.u_off) return SBD_TPB_OK;
+  if (!p.u_off || !union_ahead<T>(h, p.u_reuse, h->blk_max[blk], h->blk_max[blk + 1], rows16)) return SBD_TPB_OK;
   T **val = reinterpret_cast<T **>(sizeof(T) == 8 ? (void **)&p.u_val : (void **)&p.u_valf);
   if (!*val) {
     const size_t bytes = sizeof(T) * kBlkRows * p.u_total, smem = (n + 3) / 4 * 4 + n * 4;
@@ -1339,8 +1358,8 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
   TPB_CHECK(build_coulomb_table(h, h->pb, h->d_astr, na));
   UnionArgs ua, ub;
   if (!small_problem(h, na, nb)) {
-    TPB_CHECK(build_union<T>(h, h->pa, na, &ua));
-    TPB_CHECK(build_union<T>(h, h->pb, nb, &ub));
+    TPB_CHECK(build_union<T>(h, h->pa, na, 0, rows_aligned(nb, C, sigma, CT), &ua));
+    TPB_CHECK(build_union<T>(h, h->pb, nb, 2, rows_aligned(na, CT, sigma), &ub));
   }
 
   BlockArgs ba{};
@@ -1432,7 +1451,7 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
   TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab));
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   UnionArgs ua;
-  if (!small_problem(h, na, nb)) TPB_CHECK(build_union<T>(h, h->pa, na, &ua));
+  if (!small_problem(h, na, nb)) TPB_CHECK(build_union<T>(h, h->pa, na, 0, rows_aligned(nb, C, sigma), &ua));
   BlockArgs ba{};
   ba.u = ua;
   ba.s_off = h->ta_s.off;

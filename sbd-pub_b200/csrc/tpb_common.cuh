@@ -112,6 +112,7 @@ struct SigmaProg {
   double *u_val = nullptr;
   float *u_valf = nullptr;
   size_t u_total = 0;
+  double u_reuse = 0.0;  // doubles per entry of the list
   bool u_tried = false;
 };
 

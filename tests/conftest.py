@@ -39,6 +39,18 @@ def golden_problem(name):
                    astr=g["astr"], bstr=g["bstr"]), g, meta
 
 
+def launched_kernels(call):
+    """The names of the library's kernels that call() launches, in order (the CUDA activity trace)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as p:
+        call()
+        torch.cuda.synchronize()
+    on_gpu = [e for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    return [e.name for e in sorted(on_gpu, key=lambda e: e.time_range.start) if "sbdtpb" in e.name]
+
+
 @pytest.fixture(scope="session")
 def oracle():
     import pyoracle

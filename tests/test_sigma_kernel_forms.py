@@ -2,13 +2,13 @@
 
 Vectors whose rows are 16-byte aligned (row length a multiple of 16 bytes / element size, base
 address 16-byte aligned) take the passes that cover two 16-byte column groups per thread; a vector
-viewed one element into its buffer takes the one-group passes with scalar loads.  Both sum the same
-terms in the same order with the same roundings (fused multiply-add for the doubles terms, rounded
+viewed one element into its buffer takes passes with scalar loads, per row or by distinct ket of 8 rows;
+small problems one row per thread.  All sum the same terms in the same order with the same roundings (fused multiply-add for the doubles terms, rounded
 FP64 products for the singles and the diagonal), so sigma is bitwise equal: general form
 (convention 1, with and without accumulate) and exchange-symmetric one-pass form (convention 2)."""
 import pytest
 
-from conftest import golden_problem
+from conftest import launched_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -33,34 +33,79 @@ def _offset_copy(v):
     return view
 
 
-def _problems():
+# name -> norb, electrons and strings of each spin, and the same-spin passes that aligned and offset vectors
+# take: one row per thread below 8,192 determinants per SM whatever the rows; with few connections the
+# per-row passes of two column groups and of scalar loads; and a set between the lines of the two kinds of
+# row (1.77 doubles per distinct ket, six CTAs of the per-row passes on an SM in FP64, eight in FP32), whose
+# offset vectors take the union passes.
+FORMS = {
+    "fci12": (12, 6, 924, "sigma_block_kernel", "sigma_block_kernel"),
+    "sci24": (24, 8, 1500, "_cm_kernel", "sigma_block_kernel"),
+    "sci20": (20, 6, 2000, "_cm_kernel", "sigma_union_kernel"),
+}
+
+
+def _sampled(norb, n, count):
     import synth
-    yield "fci12", golden_problem("fci12")[0]
-    yield "sci24", synth.make_problem("sci24", nstrings=1500)
+    from sbd_tpb import Problem
+    h1, eri, core = synth.synthetic_hamiltonian(norb)
+    s = synth.sample_strings(norb, n, count)
+    return Problem(norb=norb, nelec=2 * n, core=core, h1=h1, eri_packed=eri, astr=s, bstr=s.copy())
 
 
+def _passes(names):
+    """The same-spin passes among kernel names."""
+    return [k for k in names if "sigma_" in k and "_kernel" in k and "sigma_sym_add" not in k]
+
+
+@pytest.mark.parametrize("name", sorted(FORMS))
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
-def test_aligned_and_offset_vectors_give_same_bits(dtype):
+def test_aligned_and_offset_vectors_give_same_bits(name, dtype):
     import torch
 
     import sbd_tpb
+    norb, ne, count, aligned, offset = FORMS[name]
+    prob = _sampled(norb, ne, count)
     tdt = getattr(torch, dtype)
-    vw = 16 // torch.empty(0, dtype=tdt).element_size()
-    for name, prob in _problems():
-        n = len(prob.astr)
-        assert n % vw == 0, name  # aligned rows: the two-group passes run
-        h = sbd_tpb.Handle(0)
-        h.set_problem(prob)
-        for symmetric in (False, True):
-            x = _vec(n, tdt, 5, symmetric)
-            y0 = _vec(n, tdt, 6, False)
-            for accumulate in ((False,) if symmetric else (False, True)):
-                a_out = y0.clone()
-                h.sigma_device(x, a_out, accumulate=accumulate, symmetric=symmetric)
-                u_x, u_out = _offset_copy(x), _offset_copy(y0)
-                h.sigma_device(u_x, u_out, accumulate=accumulate, symmetric=symmetric)
-                torch.cuda.synchronize()
-                assert torch.isfinite(a_out).all()
-                assert torch.equal(a_out, u_out), (name, dtype, symmetric, accumulate,
-                                                   float((a_out.double() - u_out.double()).abs().max()))
-        h.close()
+    n = len(prob.astr)
+    assert n % (16 // torch.empty(0, dtype=tdt).element_size()) == 0  # aligned rows
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    for symmetric in (False, True):
+        x = _vec(n, tdt, 5, symmetric)
+        y0 = _vec(n, tdt, 6, False)
+        for accumulate in ((False,) if symmetric else (False, True)):
+            a_out, u_out, u_x = y0.clone(), _offset_copy(y0), _offset_copy(x)
+            for want, xx, yy in ((aligned, x, a_out), (offset, u_x, u_out)):
+                ran = _passes(launched_kernels(
+                    lambda: h.sigma_device(xx, yy, accumulate=accumulate, symmetric=symmetric)))
+                assert len(ran) == (1 if symmetric else 2) and all(want in k for k in ran), ran
+            assert torch.isfinite(a_out).all()
+            assert torch.equal(a_out, u_out), (name, dtype, symmetric, accumulate,
+                                               float((a_out.double() - u_out.double()).abs().max()))
+    h.close()
+
+
+@pytest.mark.parametrize("norb, ne, count, dtype, union", [
+    (20, 6, 2000, "float64", False),  # sampled, 1.77 doubles per distinct ket, six per-row CTAs on an SM
+    (20, 6, 2000, "float32", False),
+    (20, 6, 2001, "float64", True),   # scalar rows
+    (22, 7, 4000, "float32", False),  # 1.58
+    (24, 8, 1500, "float64", False),  # 1.29
+    (24, 8, 1501, "float32", False),
+])
+def test_union_passes_run_where_they_are_ahead(norb, ne, count, dtype, union):
+    """On sampled sets the per-row passes with 16-byte rows stay ahead well above 1.5 doubles per distinct
+    ket (20 orbitals, 2,000 strings: FP64 0.39 against 0.46 ms, FP32 0.23 against 0.36)."""
+    import torch
+
+    import sbd_tpb
+    prob = _sampled(norb, ne, count)
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    x = _vec(count, getattr(torch, dtype), 5, True)
+    y = torch.empty_like(x)
+    for symmetric in (False, True):
+        ran = _passes(launched_kernels(lambda: h.sigma_device(x, y, symmetric=symmetric)))
+        assert ran and all(("sigma_union_kernel" in k) == union for k in ran), ran
+    h.close()
