@@ -15,6 +15,8 @@
 // M / (singles per string) times the multiply-adds of the direct loop, in registers and on the FP64
 // tensor pipe instead of through two shared-memory reads each.
 #include <algorithm>
+#include <bitset>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -387,51 +389,74 @@ int launch_rows(sbd_tpb_handle *h, RowArgs a, const T *C, T *sigma) {
   return SBD_TPB_OK;
 }
 
-template <typename T>
-int upload(sbd_tpb_handle *h, T **dst, const std::vector<T> &src) {
-  TPB_CUDA(cudaMalloc(dst, sizeof(T) * std::max<size_t>(1, src.size())));
-  TPB_CUDA(h2d(h, *dst, src.data(), sizeof(T) * src.size()));
-  return SBD_TPB_OK;
-}
+// Status words of the kernel's bounded waits, from one pinned page per device: pinning memory takes 1.3 ms
+// (and unpinning 0.4), as long as twenty sigmas of a small problem.  A word belongs to one handle from its
+// first program to its end; when all 1,024 of a page are taken a handle pins its own.
+class StatusPage {
+ public:
+  int *get() {
+    std::lock_guard<std::mutex> lock(m_);
+    cudaPointerAttributes at;
+    if (page_ && (cudaPointerGetAttributes(&at, page_) != cudaSuccess || at.type != cudaMemoryTypeHost))
+      page_ = nullptr;  // the program reset the device: the page went with its context
+    if (!page_ && cudaHostAlloc(&page_, sizeof(int) * kWords, cudaHostAllocMapped) == cudaSuccess) taken_.reset();
+    size_t k = 0;
+    while (k < kWords && taken_[k]) k++;
+    int *w = nullptr;
+    if (page_ && k < kWords) {
+      taken_[k] = true;
+      w = page_ + k;
+    } else if (cudaHostAlloc(&w, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+      w = nullptr;
+    }
+    cudaGetLastError();
+    if (w) *w = 0;
+    return w;
+  }
+  void put(int *w) {
+    std::lock_guard<std::mutex> lock(m_);
+    if (page_ && w >= page_ && w < page_ + kWords) taken_[w - page_] = false;
+    else cudaFreeHost(w);
+  }
+
+ private:
+  static constexpr size_t kWords = 1024;
+  std::mutex m_;
+  int *page_ = nullptr;
+  std::bitset<kWords> taken_;
+};
+constexpr int kMaxDevices = 64;
+StatusPage g_status[kMaxDevices];
 
 }  // namespace
 
 void ab_rows_free(sbd_tpb_handle *h) {
   ABRows &r = h->abr;
-  for (void *p : {(void *)r.rows, (void *)r.ent, (void *)r.pair_m, (void *)r.m_pair, (void *)r.hdr, (void *)r.prog})
-    if (p) cudaFree(p);
-  if (r.err) cudaFreeHost(r.err);
+  if (r.block) cudaFree(r.block);
+  if (r.err) g_status[h->device % kMaxDevices].put(r.err);
   r = ABRows();
 }
 
 // The row program, built once per table build; ready stays false where the direct kernel is the
 // better one or the program does not fit.
-int ab_rows_prepare(sbd_tpb_handle *h) {
+int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host) {
   ABRows &r = h->abr;
   if (r.tried) return SBD_TPB_OK;
   r.tried = true;
   const size_t na = h->astr.size(), nb = h->bstr.size(), L2 = (size_t)h->L * h->L;
   const size_t nnza = h->ta_s.nnz, nnzb = h->tb_s.nnz;
   if (!nnza || !nnzb) return SBD_TPB_OK;
-  std::vector<uint32_t> ao(na + 1), bo(nb + 1), aket(nnza), bket(nnzb);
-  std::vector<int32_t> apair(nnza), bpair(nnzb);
-  TPB_CUDA(cudaMemcpy(ao.data(), h->ta_s.off, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToHost));
-  TPB_CUDA(cudaMemcpy(bo.data(), h->tb_s.off, sizeof(uint32_t) * (nb + 1), cudaMemcpyDeviceToHost));
-  TPB_CUDA(cudaMemcpy(aket.data(), h->ta_s.ket, sizeof(uint32_t) * nnza, cudaMemcpyDeviceToHost));
-  TPB_CUDA(cudaMemcpy(apair.data(), h->pa.s_pair, sizeof(int32_t) * nnza, cudaMemcpyDeviceToHost));
-  TPB_CUDA(cudaMemcpy(bket.data(), h->tb_s.ket, sizeof(uint32_t) * nnzb, cudaMemcpyDeviceToHost));
-  TPB_CUDA(cudaMemcpy(bpair.data(), h->pb.s_pair, sizeof(int32_t) * nnzb, cudaMemcpyDeviceToHost));
+  TPB_CHECK(host.fetch(h));
+  const std::vector<uint32_t> &ao = host.ao, &bo = host.bo, &bket = host.bket;
+  const std::vector<int32_t> &bpair = host.bpair;
   auto pair_of = [](int32_t ps) { return (ps > 0 ? ps : -ps) - 1; };
   // rows of P: the unordered pairs of the beta singles, ascending
   std::vector<int32_t> pair_m(L2, -1), m_pair;
   std::vector<char> seen(L2, 0);
-  for (int32_t ps : bpair) {
-    const int pq = pair_of(ps), x = pq / h->L, y = pq % h->L;
-    seen[std::min(x, y) * h->L + std::max(x, y)] = 1;
-  }
+  for (int32_t ps : bpair) seen[pair_of(ps)] = 1;
   for (int x = 0; x < h->L; x++)
     for (int y = x; y < h->L; y++)
-      if (seen[x * h->L + y]) {
+      if (seen[x * h->L + y] || seen[y * h->L + x]) {
         pair_m[x * h->L + y] = pair_m[y * h->L + x] = (int32_t)m_pair.size();
         m_pair.push_back(x * h->L + y);
       }
@@ -447,19 +472,25 @@ int ab_rows_prepare(sbd_tpb_handle *h) {
   // a string lie above 100, where the padded products lose.
   double gemm = 0.0;
   uint32_t kmax = 0;
-  std::vector<uint32_t> rows;
   for (size_t i = 0; i < na; i++) {
     const uint32_t k = ao[i + 1] - ao[i];
-    if (k) rows.push_back((uint32_t)i);
     kmax = std::max(kmax, k);
-    gemm += (double)((k + 7) / 8 * 8) * (8.0 * r.bpp * r.passes) * (double)nb;
+    gemm += (double)((k + 7) / 8 * 8);
   }
+  gemm *= 8.0 * r.bpp * r.passes * (double)nb;
   if (gemm > 20.0 * (double)nnza * (double)nnzb) return SBD_TPB_OK;
+  std::vector<uint32_t> rows;
+  for (size_t i = 0; i < na; i++)
+    if (ao[i + 1] > ao[i]) rows.push_back((uint32_t)i);
   std::stable_sort(rows.begin(), rows.end(),
                    [&](uint32_t x, uint32_t y) { return ao[x + 1] - ao[x] > ao[y + 1] - ao[y]; });
   r.nrows = (uint32_t)rows.size();
   r.kcap = (std::min<uint32_t>(kmax, kMaxK) + 7) & ~7u;
   // alpha singles, per row ascending by the row of P of their own pair
+  std::vector<uint32_t> aket(nnza);
+  std::vector<int32_t> apair(nnza);
+  TPB_CUDA(cudaMemcpy(aket.data(), h->ta_s.ket, sizeof(uint32_t) * nnza, cudaMemcpyDeviceToHost));
+  TPB_CUDA(cudaMemcpy(apair.data(), h->pa.s_pair, sizeof(int32_t) * nnza, cudaMemcpyDeviceToHost));
   std::vector<uint2> ent(nnza);
   for (size_t e = 0; e < nnza; e++) ent[e] = make_uint2(aket[e], (uint32_t)apair[e]);
   for (size_t i = 0; i < na; i++)
@@ -528,15 +559,33 @@ int ab_rows_prepare(sbd_tpb_handle *h) {
   hdr[ncell] = make_uint4((uint32_t)prog.size(), 0, 0, 0);
   r.prog_cap = (uint32_t)cap;
   if (rows_smem(r, sizeof(double), nb, false, 2) > h->smem_optin) return SBD_TPB_OK;
-  TPB_CHECK(upload(h, &r.rows, rows));
-  TPB_CHECK(upload(h, &r.ent, ent));
-  TPB_CHECK(upload(h, &r.pair_m, pair_m));
-  TPB_CHECK(upload(h, &r.m_pair, m_pair));
-  TPB_CHECK(upload(h, &r.hdr, hdr));
-  TPB_CHECK(upload(h, &r.prog, prog));
+  // one allocation holds all of it
+  size_t bytes = 0;
+  auto part = [&](const auto &v) {
+    const size_t at = bytes;
+    bytes = (bytes + sizeof(v[0]) * v.size() + 15) & ~(size_t)15;
+    return at;
+  };
+  const size_t o_rows = part(rows), o_ent = part(ent), o_pair = part(pair_m), o_m = part(m_pair), o_hdr = part(hdr),
+               o_prog = part(prog);
+  TPB_CUDA(cudaMalloc(&r.block, bytes));
+  unsigned char *d = r.block;
+  auto place = [&](size_t at, const auto &v) { return h2d(h, d + at, v.data(), sizeof(v[0]) * v.size()); };
+  TPB_CUDA(place(o_rows, rows));
+  TPB_CUDA(place(o_ent, ent));
+  TPB_CUDA(place(o_pair, pair_m));
+  TPB_CUDA(place(o_m, m_pair));
+  TPB_CUDA(place(o_hdr, hdr));
+  TPB_CUDA(place(o_prog, prog));
   TPB_CUDA(cudaStreamSynchronize(h->stream));
-  TPB_CUDA(cudaHostAlloc(&r.err, sizeof(int), cudaHostAllocMapped));
-  *r.err = 0;
+  r.rows = reinterpret_cast<uint32_t *>(d + o_rows);
+  r.ent = reinterpret_cast<uint2 *>(d + o_ent);
+  r.pair_m = reinterpret_cast<int32_t *>(d + o_pair);
+  r.m_pair = reinterpret_cast<int32_t *>(d + o_m);
+  r.hdr = reinterpret_cast<uint4 *>(d + o_hdr);
+  r.prog = d + o_prog;
+  r.err = g_status[h->device % kMaxDevices].get();
+  if (!r.err) return fail(SBD_TPB_ERR_OOM, "alpha-beta row program: pinned status word");
   r.ready = true;
   return SBD_TPB_OK;
 }

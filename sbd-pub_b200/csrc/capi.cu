@@ -225,6 +225,7 @@ int sbd_tpb_set_strings(sbd_tpb_handle *h, const uint64_t *astr, size_t na, cons
   }
   h->astr.assign(astr, astr + na);
   h->bstr.assign(bstr, bstr + nb);
+  h->same_strings = h->astr == h->bstr;
   h->n_alpha = nea;
   h->n_beta = neb;
   TPB_CHECK(build_string_data(h));
@@ -239,6 +240,7 @@ int sbd_tpb_build_tables(sbd_tpb_handle *h) {
   TPB_CHECK(build_excitation_tables(h));
   TPB_CHECK(prepare_block_sizes(h));
   TPB_CHECK(build_sigma_programs(h));
+  TPB_CHECK(count_unions(h));
   TPB_CHECK(compute_diagonal(h));
   TPB_CHECK(ab_dense_setup(h, ab_dense_worthwhile(h) ? 1 : 0));
   TPB_CUDA(cudaStreamSynchronize(h->stream));

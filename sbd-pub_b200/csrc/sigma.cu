@@ -1098,45 +1098,19 @@ __global__ void __launch_bounds__(256)
       uval[((size_t)u0 + pos[ket[e]]) * kBlkRows + r] = val[e];
 }
 
-// The union list of a sigma program (n strings, blk: its entries of h->blk_max), built on first use per
-// problem and type; left out (u->off null) where the per-row passes are ahead, the singles have no
-// Coulomb table, or it would take more than an eighth of the free memory.
+// Shared memory of union_fill_kernel: a byte of rows and the place in the list per ket.
+inline size_t union_map_bytes(size_t n) { return (n + 3) / 4 * 4 + n * 4; }
+
+// The entries of a sigma program's union list (n strings, max_d / max_s: its largest block), built on
+// first use per problem and type; left out (u->off null) where the per-row passes are ahead or it would
+// take more than an eighth of the free memory.
 template <typename T>
-int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, int blk, bool rows16, UnionArgs *u) {
+int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, size_t max_d, size_t max_s, bool rows16, UnionArgs *u) {
   *u = UnionArgs();
-  if (!p.u_tried) {
-    p.u_tried = true;
-    const size_t smem = (n + 3) / 4 * 4 + n * 4, nblk = (n + kBlkRows - 1) / kBlkRows;
-    if (p.d->nnz == 0 || n >= (1u << 24) || smem + 1024 > h->smem_optin || (p.s->nnz && !p.jtab)) return SBD_TPB_OK;
-    uint32_t *d_cnt = nullptr;
-    std::vector<uint32_t> off(nblk + 1, 0);
-    TPB_CUDA(cudaMalloc(&d_cnt, sizeof(uint32_t) * nblk));
-    TPB_CUDA(cudaFuncSetAttribute(union_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    union_count_kernel<<<(unsigned)nblk, 256, smem, h->stream>>>(p.d->off, p.d->ket, (uint32_t)n, d_cnt);
-    h->launches++;
-    const cudaError_t e1 = cudaGetLastError();
-    const cudaError_t e2 = e1 != cudaSuccess ? e1
-                                             : cudaMemcpyAsync(off.data() + 1, d_cnt, sizeof(uint32_t) * nblk,
-                                                               cudaMemcpyDeviceToHost, h->stream);
-    const cudaError_t e3 = e2 != cudaSuccess ? e2 : cudaStreamSynchronize(h->stream);
-    cudaFree(d_cnt);
-    if (e3 != cudaSuccess) return fail(SBD_TPB_ERR_CUDA, std::string("union list: ") + cudaGetErrorString(e3));
-    size_t total = 0;
-    for (size_t b = 0; b < nblk; b++) {
-      total += off[b + 1];
-      if (total > 0xfffffff0ull) return SBD_TPB_OK;
-      off[b + 1] = (uint32_t)total;
-    }
-    p.u_reuse = (double)p.d->nnz / (double)total;
-    TPB_CUDA(cudaMalloc(&p.u_off, sizeof(uint32_t) * (nblk + 1)));
-    TPB_CUDA(h2d(h, p.u_off, off.data(), sizeof(uint32_t) * (nblk + 1)));
-    TPB_CUDA(cudaStreamSynchronize(h->stream));
-    p.u_total = total;
-  }
-  if (!p.u_off || !union_ahead<T>(h, p.u_reuse, h->blk_max[blk], h->blk_max[blk + 1], rows16)) return SBD_TPB_OK;
+  if (!p.u_off || !union_ahead<T>(h, p.u_reuse, max_d, max_s, rows16)) return SBD_TPB_OK;
   T **val = reinterpret_cast<T **>(sizeof(T) == 8 ? (void **)&p.u_val : (void **)&p.u_valf);
   if (!*val) {
-    const size_t bytes = sizeof(T) * kBlkRows * p.u_total, smem = (n + 3) / 4 * 4 + n * 4;
+    const size_t bytes = sizeof(T) * kBlkRows * p.u_total;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 8) {
       cudaGetLastError();
@@ -1149,6 +1123,7 @@ int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, int blk, bool rows16,
       return SBD_TPB_OK;
     }
     const T *src = reinterpret_cast<const T *>(sizeof(T) == 8 ? (const void *)p.d_val : (const void *)p.d_valf);
+    const size_t smem = union_map_bytes(n);
     TPB_CUDA(cudaFuncSetAttribute(union_fill_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     union_fill_kernel<T><<<(unsigned)((n + kBlkRows - 1) / kBlkRows), 256, smem, h->stream>>>(
         p.d->off, p.d->ket, src, (uint32_t)n, p.u_off, p.u_ket, *val);
@@ -1188,16 +1163,68 @@ int prepare_block_sizes(sbd_tpb_handle *h) {
   return SBD_TPB_OK;
 }
 
+// Offsets of the union list of each spin's doubles, and how many doubles share an entry, which says
+// whether the list is worth its entries (union_ahead).  Part of the table build, so that a sigma that
+// does not take the union passes pays nothing for the question (asked in the first sigma, with a buffer
+// of its own, it cost 0.3 ms at 20,000 strings, a twelfth of that call's set-up).  Identical lists share
+// alpha's.  Problems below the line of the one-row passes never ask.
+int count_unions(sbd_tpb_handle *h) {
+  const size_t na = h->astr.size(), nb = h->bstr.size();
+  if (small_problem(h, na, nb)) return SBD_TPB_OK;
+  for (int s = 0; s < (h->same_strings ? 1 : 2); s++) {
+    SigmaProg &p = s ? h->pb : h->pa;
+    const size_t n = s ? nb : na, nblk = (n + kBlkRows - 1) / kBlkRows;
+    if (p.d->nnz == 0 || n >= (1u << 24) || union_map_bytes(n) + 1024 > h->smem_optin) continue;
+    std::vector<uint32_t> off(nblk + 1, 0);
+    TPB_CUDA(cudaMallocAsync(&p.u_off, sizeof(uint32_t) * (nblk + 1), h->stream));
+    const size_t smem = (n + 3) / 4 * 4;
+    TPB_CUDA(cudaFuncSetAttribute(union_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    union_count_kernel<<<(unsigned)nblk, 256, smem, h->stream>>>(p.d->off, p.d->ket, (uint32_t)n, p.u_off + 1);
+    TPB_LAUNCHED(h);
+    TPB_CUDA(cudaMemcpyAsync(off.data() + 1, p.u_off + 1, sizeof(uint32_t) * nblk, cudaMemcpyDeviceToHost, h->stream));
+    TPB_CUDA(cudaStreamSynchronize(h->stream));
+    size_t total = 0;
+    for (size_t b = 0; b < nblk; b++) {
+      total += off[b + 1];
+      off[b + 1] = (uint32_t)total;
+    }
+    if (total > 0xfffffff0ull) continue;  // u_reuse stays 0: no union passes
+    TPB_CUDA(h2d(h, p.u_off, off.data(), sizeof(uint32_t) * (nblk + 1)));
+    TPB_CUDA(cudaStreamSynchronize(h->stream));
+    p.u_total = total;
+    p.u_reuse = (double)p.d->nnz / (double)total;
+  }
+  return SBD_TPB_OK;
+}
+
+int SinglesHost::fetch(sbd_tpb_handle *h) {
+  if (have) return SBD_TPB_OK;
+  const size_t na = h->astr.size(), nb = h->bstr.size(), nnz = h->tb_s.nnz;
+  ao.resize(na + 1);
+  bo.resize(nb + 1);
+  bket.resize(nnz);
+  bpair.resize(nnz);
+  TPB_CUDA(cudaMemcpy(ao.data(), h->ta_s.off, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToHost));
+  TPB_CUDA(cudaMemcpy(bo.data(), h->tb_s.off, sizeof(uint32_t) * (nb + 1), cudaMemcpyDeviceToHost));
+  if (nnz) {
+    TPB_CUDA(cudaMemcpy(bket.data(), h->tb_s.ket, sizeof(uint32_t) * nnz, cudaMemcpyDeviceToHost));
+    TPB_CUDA(cudaMemcpy(bpair.data(), h->pb.s_pair, sizeof(int32_t) * nnz, cudaMemcpyDeviceToHost));
+  }
+  have = true;
+  return SBD_TPB_OK;
+}
+
 // Host-side facts about the tables that size the sigma launches: the per-block table sizes
 // (prepare_block_sizes, done at table build) and, when want_ab_lists, the alpha rows and beta
 // columns that have singles (the sparse alpha-beta launch).  Computed once per table build.
-int prepare_sigma_meta(sbd_tpb_handle *h, bool want_ab_lists) {
+int prepare_sigma_meta(sbd_tpb_handle *h, bool want_ab_lists, SinglesHost &host) {
   const size_t na = h->astr.size(), nb = h->bstr.size();
   TPB_CHECK(prepare_block_sizes(h));
   if (want_ab_lists && !h->d_ab_rows && na > 0 && nb > 0) {
-    std::vector<uint32_t> ao(na + 1), bo(nb + 1), rows;
-    TPB_CUDA(cudaMemcpy(ao.data(), h->ta_s.off, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToHost));
-    TPB_CUDA(cudaMemcpy(bo.data(), h->tb_s.off, sizeof(uint32_t) * (nb + 1), cudaMemcpyDeviceToHost));
+    TPB_CHECK(host.fetch(h));
+    const std::vector<uint32_t> &ao = host.ao, &bo = host.bo, &bket = host.bket;
+    const std::vector<int32_t> &bpair = host.bpair;
+    std::vector<uint32_t> rows;
     uint32_t kmax = 0;
     for (size_t i = 0; i < na; i++)
       if (ao[i + 1] > ao[i]) {
@@ -1212,12 +1239,6 @@ int prepare_sigma_meta(sbd_tpb_handle *h, bool want_ab_lists) {
     // beta program: columns with singles and their entries, packed so a thread needs one load
     // per column and one per entry
     const size_t nnz = bo[nb];
-    std::vector<uint32_t> bket(std::max<size_t>(1, nnz));
-    std::vector<int32_t> bpair(std::max<size_t>(1, nnz));
-    if (nnz) {
-      TPB_CUDA(cudaMemcpy(bket.data(), h->tb_s.ket, sizeof(uint32_t) * nnz, cudaMemcpyDeviceToHost));
-      TPB_CUDA(cudaMemcpy(bpair.data(), h->pb.s_pair, sizeof(int32_t) * nnz, cudaMemcpyDeviceToHost));
-    }
     // columns ordered by their number of singles (most first, then by column), entries regrouped
     // in that order: the lanes of a warp take consecutive columns and loop over their singles, so
     // similar counts side by side keep the lanes busy (in column order ~30 % of the lane
@@ -1350,16 +1371,21 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
     h->ct_bytes = n * sizeof(double);
   }
   T *CT = reinterpret_cast<T *>(h->d_ct);
-  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h));
+  SinglesHost host;
+  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h, host));
   const bool rows_ab = h->abr.ready && !dense_ab;
-  TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab));
+  TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab, host));
   // per-pair Coulomb sums of the singles over the other spin's strings (built once per problem)
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   TPB_CHECK(build_coulomb_table(h, h->pb, h->d_astr, na));
   UnionArgs ua, ub;
   if (!small_problem(h, na, nb)) {
-    TPB_CHECK(build_union<T>(h, h->pa, na, 0, rows_aligned(nb, C, sigma, CT), &ua));
-    TPB_CHECK(build_union<T>(h, h->pb, nb, 2, rows_aligned(na, CT, sigma), &ub));
+    const uint32_t *m = h->blk_max;
+    // (the union passes read the singles' Coulomb sums from their table)
+    if (h->pa.jtab || !h->ta_s.nnz)
+      TPB_CHECK(build_union<T>(h, h->pa, na, m[0], m[1], rows_aligned(nb, C, sigma, CT), &ua));
+    if (h->pb.jtab || !h->tb_s.nnz)
+      TPB_CHECK(build_union<T>(h, h->same_strings ? h->pa : h->pb, nb, m[2], m[3], rows_aligned(na, CT, sigma), &ub));
   }
 
   BlockArgs ba{};
@@ -1443,15 +1469,17 @@ template <typename T>
 int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T *const *S, int m,
                   int slot) {
   const uint32_t na = (uint32_t)h->astr.size(), nb = (uint32_t)h->bstr.size();
-  if (na != nb || h->astr != h->bstr)
+  if (!h->same_strings)
     return fail(SBD_TPB_ERR_STATE, "symmetric sigma needs identical alpha and beta strings");
   const bool dense_ab = h->ab.enabled && sizeof(T) == 4 && h->ab.tc_ready;
-  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h));
+  SinglesHost host;
+  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h, host));
   const bool rows_ab = h->abr.ready && !dense_ab;
-  TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab));
+  TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab, host));
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   UnionArgs ua;
-  if (!small_problem(h, na, nb)) TPB_CHECK(build_union<T>(h, h->pa, na, 0, rows_aligned(nb, C, sigma), &ua));
+  if (!small_problem(h, na, nb) && (h->pa.jtab || !h->ta_s.nnz))
+    TPB_CHECK(build_union<T>(h, h->pa, na, h->blk_max[0], h->blk_max[1], rows_aligned(nb, C, sigma), &ua));
   BlockArgs ba{};
   ba.u = ua;
   ba.s_off = h->ta_s.off;
@@ -1506,7 +1534,7 @@ template int sigma_sep_sym<float>(sbd_tpb_handle *, const float *, float *, doub
 template <typename T>
 int sigma_sep_given_ct(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, T *CT) {
   const uint32_t na = (uint32_t)h->astr.size(), nb = (uint32_t)h->bstr.size();
-  TPB_CHECK(prepare_sigma_meta(h, false));
+  TPB_CHECK(prepare_block_sizes(h));
   BlockArgs ba{};
   ba.s_off = h->ta_s.off;
   ba.s_ket = h->ta_s.ket;

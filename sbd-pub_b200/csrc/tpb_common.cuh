@@ -107,13 +107,13 @@ struct SigmaProg {
   int32_t *pmap = nullptr;
   uint32_t npair = 0;
   bool jtab_tried = false;  // built, or found too large, once per program
-  // doubles of each 8-row block by distinct ket (build_union, sigma.cu): dense tables only
+  // doubles of each 8-row block by distinct ket (sigma.cu): list offsets and u_reuse, the doubles per
+  // entry, from count_unions; the entries from build_union, where the union passes run
   uint32_t *u_off = nullptr, *u_ket = nullptr;
   double *u_val = nullptr;
   float *u_valf = nullptr;
   size_t u_total = 0;
-  double u_reuse = 0.0;  // doubles per entry of the list
-  bool u_tried = false;
+  double u_reuse = 0.0;
 };
 
 // Dense-path data for the alpha-beta term as gather -> (pq|rs) contraction -> scatter.
@@ -138,6 +138,7 @@ struct ABDense {
 // blocks of ket columns, and the alpha singles in the order the symmetric form needs.
 struct ABRows {
   bool tried = false, ready = false;
+  unsigned char *block = nullptr;                // the one allocation that the arrays below lie in
   uint32_t *rows = nullptr;                      // alpha rows with singles, most singles first
   uint2 *ent = nullptr;                          // alpha singles (ket, +-(pair + 1))
   int32_t *pair_m = nullptr, *m_pair = nullptr;  // pair <-> row of the product
@@ -146,6 +147,14 @@ struct ABRows {
   int M = 0, passes = 0, bpp = 0;
   uint32_t nrows = 0, nchunks = 0, kcap = 0, prog_cap = 0;
   int *err = nullptr;  // status of the kernel's bounded waits (pinned host memory it writes to)
+};
+
+// Host copies of the singles tables that the alpha-beta set-up reads, fetched once for all of it.
+struct SinglesHost {
+  bool have = false;
+  std::vector<uint32_t> ao, bo, bket;  // offsets of both spins, kets of the beta singles
+  std::vector<int32_t> bpair;          // +-(pair + 1) of the beta singles
+  int fetch(sbd_tpb_handle *h);
 };
 
 }  // namespace sbdtpb
@@ -173,6 +182,7 @@ struct sbd_tpb_handle {
   std::vector<double> h1;          // L*L
   std::vector<double> eri_packed;  // packed store
   std::vector<uint64_t> astr, bstr;
+  bool same_strings = false;  // astr == bstr
   int n_alpha = 0, n_beta = 0;
   bool have_ham = false, have_strings = false, have_tables = false;
 
@@ -261,6 +271,8 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
                   int slot = 0);
 // per-block table sizes of the sigma launches, read back once per table build (blk_max, blk_for)
 int prepare_block_sizes(sbd_tpb_handle *h);
+// distinct kets of each row block of the doubles, once per table build (SigmaProg::u_off, u_reuse)
+int count_unions(sbd_tpb_handle *h);
 int reorder_sign_apply_f64(sbd_tpb_handle *h, const double *x, double *y);
 int reorder_sign_apply_f32(sbd_tpb_handle *h, const float *x, float *y);
 // ab_dense.cu: alpha-beta term as gather -> dense (pq|rs) contraction -> scatter
@@ -269,7 +281,7 @@ bool ab_dense_worthwhile(sbd_tpb_handle *h);
 template <typename T>
 int ab_dense_apply(sbd_tpb_handle *h, const T *C, T *sigma, double scale = 1.0);
 // ab_rows.cu: alpha-beta term of densely connected sets, one tensor-core product per alpha row
-int ab_rows_prepare(sbd_tpb_handle *h);
+int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host);
 void ab_rows_free(sbd_tpb_handle *h);
 int ab_rows_check(sbd_tpb_handle *h);  // status of the launches before the last synchronisation
 template <typename T>

@@ -39,16 +39,22 @@ def golden_problem(name):
                    astr=g["astr"], bstr=g["bstr"]), g, meta
 
 
-def launched_kernels(call):
-    """The names of the library's kernels that call() launches, in order (the CUDA activity trace)."""
+def traced(call):
+    """(CUDA runtime calls, GPU activities) of call(): their names, each in order of time."""
     import torch
     from torch.profiler import ProfilerActivity, profile
     torch.cuda.synchronize()
     with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as p:
         call()
         torch.cuda.synchronize()
-    on_gpu = [e for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
-    return [e.name for e in sorted(on_gpu, key=lambda e: e.time_range.start) if "sbdtpb" in e.name]
+    at = sorted(p.events(), key=lambda e: e.time_range.start)
+    cuda = torch.autograd.DeviceType.CUDA
+    return [e.name for e in at if e.device_type != cuda], [e.name for e in at if e.device_type == cuda]
+
+
+def launched_kernels(call):
+    """The names of the library's kernels that call() launches, in order."""
+    return [k for k in traced(call)[1] if "sbdtpb" in k]
 
 
 @pytest.fixture(scope="session")
