@@ -300,7 +300,8 @@ SBD_TPB_API int sbd_tpb_last_sigma_kernels(sbd_tpb_handle *h, double *ms, int ma
 SBD_TPB_API uint64_t sbd_tpb_kernel_launches(sbd_tpb_handle *h);
 
 /* Release the handle's cached work memory: the Davidson N-vectors kept between solves, the
- * sigma C^T staging and the sign-conversion vectors.  Tables, diagonal and the problem stay;
+ * sigma C^T staging, the sign-conversion vectors and the doubles regrouped by distinct ket (densely
+ * connected sets).  Tables, diagonal and the problem stay;
  * the next call that needs the work memory allocates it again.  No counterpart in the
  * reference, whose solver frees its vectors at the end of each call. */
 SBD_TPB_API int sbd_tpb_release_work(sbd_tpb_handle *h);

@@ -219,7 +219,7 @@ int ab_dense_apply(sbd_tpb_handle *h, const T *C, T *sigma, double scale) {
     if (h->d_ab_work) cudaFree(h->d_ab_work);
     h->d_ab_work = nullptr;
     h->ab_work_bytes = 0;
-    TPB_CUDA(cudaMalloc(&h->d_ab_work, need));
+    TPB_CHECK(dev_alloc(h, need, &h->d_ab_work));
     h->ab_work_bytes = need;
   }
   const int grid = h->num_sms * 8;

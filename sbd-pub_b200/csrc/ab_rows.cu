@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <bitset>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -437,12 +438,9 @@ void ab_rows_free(sbd_tpb_handle *h) {
   r = ABRows();
 }
 
-// The row program, built once per table build; ready stays false where the direct kernel is the
-// better one or the program does not fit.
-int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host) {
+// The row program; ready stays false where the direct kernel is the better one or the program does not fit.
+static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
   ABRows &r = h->abr;
-  if (r.tried) return SBD_TPB_OK;
-  r.tried = true;
   const size_t na = h->astr.size(), nb = h->bstr.size(), L2 = (size_t)h->L * h->L;
   const size_t nnza = h->ta_s.nnz, nnzb = h->tb_s.nnz;
   if (!nnza || !nnzb) return SBD_TPB_OK;
@@ -568,6 +566,9 @@ int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host) {
   };
   const size_t o_rows = part(rows), o_ent = part(ent), o_pair = part(pair_m), o_m = part(m_pair), o_hdr = part(hdr),
                o_prog = part(prog);
+  size_t free_b = 0, total_b = 0;
+  TPB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  if (bytes > free_b / 8) return SBD_TPB_OK;
   TPB_CUDA(cudaMalloc(&r.block, bytes));
   unsigned char *d = r.block;
   auto place = [&](size_t at, const auto &v) { return h2d(h, d + at, v.data(), sizeof(v[0]) * v.size()); };
@@ -587,6 +588,23 @@ int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host) {
   r.err = g_status[h->device % kMaxDevices].get();
   if (!r.err) return fail(SBD_TPB_ERR_OOM, "alpha-beta row program: pinned status word");
   r.ready = true;
+  return SBD_TPB_OK;
+}
+
+// Builds the program once per problem.  Memory that runs short, the host's or the device's, leaves the direct
+// kernel to do the term.
+int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host) {
+  if (h->abr.tried) return SBD_TPB_OK;
+  int rc;
+  try {
+    rc = build_program(h, host);
+  } catch (const std::bad_alloc &) {
+    rc = SBD_TPB_ERR_OOM;
+  }
+  if (!h->abr.ready) ab_rows_free(h);
+  h->abr.tried = true;
+  if (rc != SBD_TPB_ERR_OOM) return rc;
+  cudaGetLastError();
   return SBD_TPB_OK;
 }
 

@@ -48,15 +48,15 @@ int use_device(sbd_tpb_handle *h) {
 
 int ensure_tmp64(sbd_tpb_handle *h) {
   const size_t n = h->ndet();
-  if (!h->d_tmp64) TPB_CUDA(cudaMalloc(&h->d_tmp64, sizeof(double) * n));
-  if (!h->d_tmp64b) TPB_CUDA(cudaMalloc(&h->d_tmp64b, sizeof(double) * n));
+  if (!h->d_tmp64) TPB_CHECK(dev_alloc(h, &h->d_tmp64, n));
+  if (!h->d_tmp64b) TPB_CHECK(dev_alloc(h, &h->d_tmp64b, n));
   return SBD_TPB_OK;
 }
 
 int ensure_tmp32(sbd_tpb_handle *h) {
   const size_t n = h->ndet();
-  if (!h->d_tmp32) TPB_CUDA(cudaMalloc(&h->d_tmp32, sizeof(float) * n));
-  if (!h->d_tmp32b) TPB_CUDA(cudaMalloc(&h->d_tmp32b, sizeof(float) * n));
+  if (!h->d_tmp32) TPB_CHECK(dev_alloc(h, &h->d_tmp32, n));
+  if (!h->d_tmp32b) TPB_CHECK(dev_alloc(h, &h->d_tmp32b, n));
   return SBD_TPB_OK;
 }
 
@@ -557,6 +557,7 @@ int sbd_tpb_release_work(sbd_tpb_handle *h) {
   if (h->d_ct) cudaFree(h->d_ct);
   h->d_ct = nullptr;
   h->ct_bytes = 0;
+  free_unions(h);
   return SBD_TPB_OK;
 }
 

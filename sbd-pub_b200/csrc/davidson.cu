@@ -229,7 +229,7 @@ int run_typed(sbd_tpb_handle *h, const sbd_tpb_params *prm, const double *W0, do
         recording = true;
         if (ib == 0) {
           float *c0 = nullptr;
-          TPB_CUDA(cudaMalloc(&c0, sizeof(float) * n));
+          TPB_CHECK(dev_alloc(h, &c0, n));
           rec->owned.push_back(c0);
           TPB_CHECK((convert_vec<T, float>(h, S[0].p, c0, n)));
           rec->vec.push_back(c0);
@@ -237,7 +237,7 @@ int run_typed(sbd_tpb_handle *h, const sbd_tpb_params *prm, const double *W0, do
           rec_cycle.assign(1, (int)rec->vec.size() - 1);
         }
         float *dk = nullptr;
-        TPB_CUDA(cudaMalloc(&dk, sizeof(float) * n));
+        TPB_CHECK(dev_alloc(h, &dk, n));
         rec->owned.push_back(dk);
         rec->d.push_back(dk);
         TPB_CHECK((convert_vec<T, float>(h, tnext, dk, n)));
@@ -334,7 +334,7 @@ int run_typed(sbd_tpb_handle *h, const sbd_tpb_params *prm, const double *W0, do
         f[ib + 1] = 1.0 / std::sqrt(tt);
         if (recording) {
           float *dp = nullptr;
-          TPB_CUDA(cudaMalloc(&dp, sizeof(float) * n));
+          TPB_CHECK(dev_alloc(h, &dp, n));
           rec->owned.push_back(dp);
           TPB_CHECK((convert_vec<T, float>(h, tnext, dp, n)));
           rec->vec.push_back(dp);
@@ -488,6 +488,14 @@ int pool_get(sbd_tpb_handle *h, size_t bytes, void **out) {
   if (cudaMalloc(out, bytes) == cudaSuccess) return SBD_TPB_OK;
   cudaGetLastError();
   pool_clear(h);
+  return dev_alloc(h, bytes, out);
+}
+
+int dev_alloc(sbd_tpb_handle *h, size_t bytes, void **out) {
+  *out = nullptr;
+  if (cudaMalloc(out, bytes) == cudaSuccess) return SBD_TPB_OK;
+  cudaGetLastError();
+  free_unions(h);
   TPB_CUDA(cudaMalloc(out, bytes));
   return SBD_TPB_OK;
 }

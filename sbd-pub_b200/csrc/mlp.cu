@@ -1187,7 +1187,7 @@ int precond_collect(sbd_tpb_precond *p, sbd_tpb_handle *h, const sbd_tpb_params 
   TPB_CHECK(ensure_occ_windows(h));
   DavRecord rec;
   double *Psi = nullptr;
-  TPB_CUDA(cudaMalloc(&Psi, sizeof(double) * h->ndet()));
+  TPB_CHECK(dev_alloc(h, &Psi, h->ndet()));
   double E = 0.0;
   // a run with the learned correction collects pairs along the learned solver's own trajectory
   int rc = davidson_record(h, prm, &rec, Psi, &E, prm->preconditioner == SBD_TPB_PRECOND_LEARNED ? p : nullptr);

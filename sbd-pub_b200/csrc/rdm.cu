@@ -382,8 +382,8 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
     // each string's orbitals in the order the full pass below adds them
     if (!density) return SBD_TPB_OK;
     double *d_rho = nullptr, *d_cp = nullptr;
-    TPB_CUDA(cudaMalloc(&d_rho, sizeof(double) * ((size_t)na + nb)));
-    TPB_CUDA(cudaMalloc(&d_cp, sizeof(double) * (size_t)nca * nb));
+    TPB_CHECK(dev_alloc(h, &d_rho, ((size_t)na + nb)));
+    TPB_CHECK(dev_alloc(h, &d_cp, (size_t)nca * nb));
     rdm_rowsum_kernel<<<na, kRdmThreads, 0, h->stream>>>(W, nb, d_rho);
     TPB_LAUNCHED(h);
     dim3 gridc((nb + 255) / 256, nca);
@@ -412,11 +412,11 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
   Rdm R(L);
   // ---- diagonal part (deterministic: fixed summation order throughout)
   double *d_rho_a = nullptr, *d_rho_b = nullptr, *d_Y = nullptr, *d_Mp = nullptr, *d_cp = nullptr;
-  TPB_CUDA(cudaMalloc(&d_rho_a, sizeof(double) * na));
-  TPB_CUDA(cudaMalloc(&d_rho_b, sizeof(double) * nb));
-  TPB_CUDA(cudaMalloc(&d_Y, sizeof(double) * (size_t)na * L));
-  TPB_CUDA(cudaMalloc(&d_Mp, sizeof(double) * (size_t)nca * L * L));
-  TPB_CUDA(cudaMalloc(&d_cp, sizeof(double) * (size_t)nca * nb));
+  TPB_CHECK(dev_alloc(h, &d_rho_a, na));
+  TPB_CHECK(dev_alloc(h, &d_rho_b, nb));
+  TPB_CHECK(dev_alloc(h, &d_Y, (size_t)na * L));
+  TPB_CHECK(dev_alloc(h, &d_Mp, (size_t)nca * L * L));
+  TPB_CHECK(dev_alloc(h, &d_cp, (size_t)nca * nb));
   rdm_row_kernel<<<na, kRdmThreads, 0, h->stream>>>(W, h->d_bstr, nb, L, d_rho_a, d_Y);
   TPB_LAUNCHED(h);
   {
@@ -472,9 +472,9 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
     TPB_CHECK(fetch(h, h->tb_d, nb, bd));
     double *d_WT = nullptr, *d_T0 = nullptr, *d_Tq = nullptr;
     const size_t maxp = std::max({h->ta_s.nnz, h->ta_d.nnz, h->tb_s.nnz, h->tb_d.nnz, (size_t)1});
-    TPB_CUDA(cudaMalloc(&d_WT, sizeof(double) * n));
-    TPB_CUDA(cudaMalloc(&d_T0, sizeof(double) * maxp));
-    TPB_CUDA(cudaMalloc(&d_Tq, sizeof(double) * maxp * L));
+    TPB_CHECK(dev_alloc(h, &d_WT, n));
+    TPB_CHECK(dev_alloc(h, &d_T0, maxp));
+    TPB_CHECK(dev_alloc(h, &d_Tq, maxp * L));
     {
       dim3 grid((nb + 31) / 32, (na + 31) / 32), block(32, 8);
       transpose_kernel<<<grid, block, 0, h->stream>>>(W, d_WT, na, nb);
@@ -516,9 +516,9 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
           ord[t] = single_sign(str[i], cr, an) > 0 ? (int32_t)e + 1 : -((int32_t)e + 1);
           bra[t] = str[i];
         }
-      TPB_CUDA(cudaMalloc(&lb.seg, sizeof(uint32_t) * seg.size()));
-      TPB_CUDA(cudaMalloc(&lb.ord, sizeof(int32_t) * std::max<size_t>(1, w)));
-      TPB_CUDA(cudaMalloc(&lb.bra, sizeof(uint64_t) * std::max<size_t>(1, w)));
+      TPB_CHECK(dev_alloc(h, &lb.seg, seg.size()));
+      TPB_CHECK(dev_alloc(h, &lb.ord, std::max<size_t>(1, w)));
+      TPB_CHECK(dev_alloc(h, &lb.bra, std::max<size_t>(1, w)));
       TPB_CUDA(h2d(h, lb.seg, seg.data(), sizeof(uint32_t) * seg.size()));
       TPB_CUDA(h2d(h, lb.ord, ord.data(), sizeof(int32_t) * w));
       TPB_CUDA(h2d(h, lb.bra, bra.data(), sizeof(uint64_t) * w));
@@ -533,7 +533,7 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
       out.resize((size_t)nl * width);
       if (!nl) return SBD_TPB_OK;
       double *d_out = nullptr;
-      TPB_CUDA(cudaMalloc(&d_out, sizeof(double) * out.size()));
+      TPB_CHECK(dev_alloc(h, &d_out, out.size()));
       if (occ) {
         rdm_label_occ_kernel<<<nl, 64, 0, h->stream>>>(X, lb.bra, lb.seg, lb.ord, d_out);
       } else {
@@ -630,10 +630,10 @@ int rdm_sep(sbd_tpb_handle *h, const double *W, double *one, double *two, double
       uint32_t *d_abra = nullptr, *d_bbra = nullptr;
       int32_t *d_blab = nullptr;
       double *d_X = nullptr;
-      TPB_CUDA(cudaMalloc(&d_abra, sizeof(uint32_t) * abra.size()));
-      TPB_CUDA(cudaMalloc(&d_bbra, sizeof(uint32_t) * bbra.size()));
-      TPB_CUDA(cudaMalloc(&d_blab, sizeof(int32_t) * blab.size()));
-      TPB_CUDA(cudaMalloc(&d_X, sizeof(double) * h->ta_s.nnz * L2));
+      TPB_CHECK(dev_alloc(h, &d_abra, abra.size()));
+      TPB_CHECK(dev_alloc(h, &d_bbra, bbra.size()));
+      TPB_CHECK(dev_alloc(h, &d_blab, blab.size()));
+      TPB_CHECK(dev_alloc(h, &d_X, h->ta_s.nnz * L2));
       TPB_CUDA(h2d(h, d_abra, abra.data(), sizeof(uint32_t) * abra.size()));
       TPB_CUDA(h2d(h, d_bbra, bbra.data(), sizeof(uint32_t) * bbra.size()));
       TPB_CUDA(h2d(h, d_blab, blab.data(), sizeof(int32_t) * blab.size()));

@@ -1116,10 +1116,9 @@ int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, size_t max_d, size_t 
       cudaGetLastError();
       return SBD_TPB_OK;
     }
-    if (!p.u_ket) TPB_CUDA(cudaMalloc(&p.u_ket, sizeof(uint32_t) * p.u_total));
-    if (cudaMalloc(val, bytes) != cudaSuccess) {
+    if ((!p.u_ket && cudaMalloc(&p.u_ket, sizeof(uint32_t) * p.u_total) != cudaSuccess) ||
+        cudaMalloc(val, bytes) != cudaSuccess) {
       cudaGetLastError();
-      *val = nullptr;
       return SBD_TPB_OK;
     }
     const T *src = reinterpret_cast<const T *>(sizeof(T) == 8 ? (const void *)p.d_val : (const void *)p.d_valf);
@@ -1133,6 +1132,18 @@ int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, size_t max_d, size_t 
   u->ket = p.u_ket;
   u->val = *val;
   return SBD_TPB_OK;
+}
+
+// The entries of the union lists given back (the offsets stay, the next sigma builds them again).
+void free_unions(sbd_tpb_handle *h) {
+  cudaStreamSynchronize(h->stream);
+  for (SigmaProg *p : {&h->pa, &h->pb}) {
+    for (void *q : {(void *)p->u_ket, (void *)p->u_val, (void *)p->u_valf})
+      if (q) cudaFree(q);
+    p->u_ket = nullptr;
+    p->u_val = nullptr;
+    p->u_valf = nullptr;
+  }
 }
 
 // Most entries of any kBlkRows-row block of a CSR table of n rows (shared-memory staging size).
@@ -1367,7 +1378,7 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
     if (h->d_ct) cudaFree(h->d_ct);
     h->d_ct = nullptr;
     h->ct_bytes = 0;
-    TPB_CUDA(cudaMalloc(&h->d_ct, n * sizeof(double)));
+    TPB_CHECK(dev_alloc(h, n * sizeof(double), &h->d_ct));
     h->ct_bytes = n * sizeof(double);
   }
   T *CT = reinterpret_cast<T *>(h->d_ct);

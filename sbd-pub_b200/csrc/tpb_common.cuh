@@ -271,6 +271,7 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
                   int slot = 0);
 // per-block table sizes of the sigma launches, read back once per table build (blk_max, blk_for)
 int prepare_block_sizes(sbd_tpb_handle *h);
+void free_unions(sbd_tpb_handle *h);
 // distinct kets of each row block of the doubles, once per table build (SigmaProg::u_off, u_reuse)
 int count_unions(sbd_tpb_handle *h);
 int reorder_sign_apply_f64(sbd_tpb_handle *h, const double *x, double *y);
@@ -293,6 +294,13 @@ int multi_dot(sbd_tpb_handle *h, const T *const *X, int k, const T *y, size_t n,
 // rdm.cu
 // W: device FP64 vector in the separated convention; outputs are host arrays (any may be null):
 // one [2L^2], two [4L^4] in the reference layouts, density [2L].
+// cudaMalloc that, where memory is short, gives the union lists back (they are built when there is room
+// for them, before what is allocated here) and tries again
+int dev_alloc(sbd_tpb_handle *h, size_t bytes, void **out);
+template <typename T>
+int dev_alloc(sbd_tpb_handle *h, T **out, size_t count) {
+  return dev_alloc(h, sizeof(T) * count, reinterpret_cast<void **>(out));
+}
 // vector pool (davidson.cu): a block of at least `bytes` (reused if one of at most twice the size
 // is free, else cudaMalloc, emptying the pool and retrying once if memory is short), its return,
 // and the release of every kept block
