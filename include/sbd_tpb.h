@@ -9,6 +9,14 @@
  * SBD_TPB_ERR_* code); sbd_tpb_last_error() gives the message of the calling thread's last
  * failure.  No entry point throws or exits the process.
  *
+ * Device buffers.  A handle works on a non-blocking stream of its own (sbd_tpb_stream).  Calls that read
+ * or write a caller's device buffer first order that stream behind what is queued on the legacy default
+ * stream at that moment (and so behind blocking streams, which it waits for): buffers written by plain
+ * launches, thrust or torch's default stream need no synchronisation before the call.  Work on other
+ * non-blocking streams, and calls made while the handle's or a blocking stream is capturing, are the
+ * caller's to order.  When a call returns its device output is complete, except sbd_tpb_sigma_noalloc's,
+ * which is queued on the handle's stream.
+ *
  * The reference interfaces each entry point replaces are cited as file:line inside ncsa/sbd-pub.
  */
 #ifndef SBD_TPB_H

@@ -25,6 +25,27 @@ int fail(int code, const std::string &msg) {
   return code;
 }
 
+// Every entry point that reads or writes a caller's device buffer starts with this.  Such buffers are usually
+// written (or, from a caching allocator, still read) by work the caller queued on the legacy default
+// stream, where torch and plain launches go and which the handle's non-blocking stream does not wait for
+// by itself: a sigma called right behind the kernel that makes its input read it half written.  The wait is
+// on the device, for what is queued so far; the legacy stream in turn waits for the blocking streams, so
+// work of theirs that is queued already is waited for too.  While the handle's stream, or one that blocks
+// on the legacy stream, is capturing (the queries say so without disturbing the capture) ordering stays
+// with the caller, as it does for work on other non-blocking streams.  About 2 us.
+int wait_for_caller(sbd_tpb_handle *h) {
+  for (cudaStream_t s : {h->stream, cudaStreamLegacy}) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return SBD_TPB_OK;
+    }
+  }
+  TPB_CUDA(cudaEventRecord(h->ev_in, cudaStreamLegacy));
+  TPB_CUDA(cudaStreamWaitEvent(h->stream, h->ev_in, 0));
+  return SBD_TPB_OK;
+}
+
 cudaError_t h2d(sbd_tpb_handle *h, void *dst, const void *src, size_t bytes) {
   return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream) : cudaSuccess;
 }
@@ -57,23 +78,6 @@ int ensure_tmp32(sbd_tpb_handle *h) {
   const size_t n = h->ndet();
   if (!h->d_tmp32) TPB_CHECK(dev_alloc(h, &h->d_tmp32, n));
   if (!h->d_tmp32b) TPB_CHECK(dev_alloc(h, &h->d_tmp32b, n));
-  return SBD_TPB_OK;
-}
-
-// Device vectors are usually written by work the caller queued on the legacy default stream (where
-// torch and plain launches go), which the handle's non-blocking stream does not wait for by itself: a
-// sigma called right behind the kernel that makes its input read it half written.  The wait is on the
-// device, for what is queued so far; while a stream that blocks on the legacy one is capturing (the
-// query says so without disturbing the capture) ordering stays with the caller, as it does for
-// vectors made on other streams.
-int wait_for_caller(sbd_tpb_handle *h) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return SBD_TPB_OK;
-  }
-  TPB_CUDA(cudaEventRecord(h->ev_in, cudaStreamLegacy));
-  TPB_CUDA(cudaStreamWaitEvent(h->stream, h->ev_in, 0));
   return SBD_TPB_OK;
 }
 
@@ -275,6 +279,7 @@ int sbd_tpb_diagonal(sbd_tpb_handle *h, double *hii, int mem) {
   TPB_HANDLE(h);
   if (!h->have_tables) return fail(SBD_TPB_ERR_STATE, "tables not built");
   if (!hii) return fail(SBD_TPB_ERR_INVALID, "null output");
+  if (mem == SBD_TPB_DEVICE) TPB_CHECK(wait_for_caller(h));
   TPB_CUDA(cudaMemcpyAsync(hii, h->d_hii, sizeof(double) * h->ndet(),
                            mem == SBD_TPB_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                            h->stream));
@@ -405,6 +410,7 @@ int sbd_tpb_rdm(sbd_tpb_handle *h, const double *W, double *one, double *two, in
   const size_t n = h->ndet();
   TPB_CHECK(ensure_tmp64(h));
   if (mem == SBD_TPB_DEVICE) {
+    TPB_CHECK(wait_for_caller(h));
     TPB_CHECK(reorder_sign_apply_f64(h, W, h->d_tmp64));
   } else {
     TPB_CUDA(cudaMemcpyAsync(h->d_tmp64b, W, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
@@ -462,7 +468,10 @@ int sbd_tpb_carryover_strings(sbd_tpb_handle *h, const double *W, int mem, sbd_t
   TPB_HANDLE(h);
   if (!h->have_strings) return fail(SBD_TPB_ERR_STATE, "strings not set");
   if (!W || !co) return fail(SBD_TPB_ERR_INVALID, "null vector/carry-over record");
-  if (mem == SBD_TPB_DEVICE) return carryover_device(h, W, co);
+  if (mem == SBD_TPB_DEVICE) {
+    TPB_CHECK(wait_for_caller(h));
+    return carryover_device(h, W, co);
+  }
   TPB_CHECK(ensure_tmp64(h));
   TPB_CUDA(cudaMemcpyAsync(h->d_tmp64, W, sizeof(double) * h->ndet(), cudaMemcpyHostToDevice, h->stream));
   return carryover_device(h, h->d_tmp64, co);

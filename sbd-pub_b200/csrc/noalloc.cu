@@ -81,6 +81,7 @@ extern "C" int sbd_tpb_sigma_noalloc(sbd_tpb_handle *h, const void *C, void *sig
   TPB_CUDA(cudaSetDevice(h->device));
   void *scratch = nullptr;
   TPB_CHECK(scratch_for_device(h->device, &scratch));
+  TPB_CHECK(wait_for_caller(h));
   if (dtype == 0)
     TPB_CHECK(sigma_sep_given_ct<double>(h, (const double *)C, (double *)sigma, accumulate,
                                          (double *)scratch));

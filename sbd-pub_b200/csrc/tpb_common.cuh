@@ -51,6 +51,8 @@ int fail(int code, const std::string &msg);
     if (rc_ != SBD_TPB_OK) return rc_; \
   } while (0)
 
+// Orders h->stream behind the work a caller queued on the legacy stream (capi.cu).
+int wait_for_caller(sbd_tpb_handle *h);
 // Host -> device copy ordered before what h->stream runs next.  (cudaMemcpy runs on the legacy stream and may
 // return while a pageable source is only staged; the handle's stream is non-blocking and would not wait for
 // it.)  Functions whose sources are locals synchronise the stream once after their last copy.
