@@ -12,6 +12,8 @@ CASES = {  # norb, (alpha electrons, strings), (beta electrons, strings)
     "unequal": (12, (4, 70), (3, 41)),
     "wide": (40, (3, 60), (2, 33)),        # 1,600 columns of label sums: several blocks of threads
     "one_string": (8, (3, 1), (4, 30)),    # no alpha singles at all
+    # 8 orbitals: doubles are summed per label from 257 of them, placed one by one below
+    "summed_and_placed": (8, (4, 40), (4, 18)),
 }
 
 
