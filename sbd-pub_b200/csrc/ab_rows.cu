@@ -70,6 +70,13 @@ struct RowArgs {
   int *err;               // pinned host memory: set when a wait expired
 };
 
+// Sums of rows that do not fit in shared memory (not kSig).
+struct RowScratch {
+  void *rows;       // [slots][nb]
+  uint32_t *taken;  // [slots] whether a CTA has the row
+  uint32_t slots;   // as many as CTAs are resident at a time
+};
+
 __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
 }
@@ -115,10 +122,16 @@ struct Bars {
 // 64-bit sums in another order went down (FP64 2.5e-16 -> 1.4e-16, FP32 6.8e-8 -> 4.1e-8 of sigma's norm).
 //
 // Shared memory: Bars, [kStages][kcap][32] of C, [pbufs][8 bpp][32] of P, per gather warp
-// [2][prog_cap] of its program, and (kSig) one sigma row.
+// [2][prog_cap] of its program, and (kSig) one row of sums.  Rows of sums that do not fit (FP64 from about 10,000
+// columns, FP32 35,000) lie in scratch rows, one per resident CTA, which stay in L2.  They are summed from zero
+// too: added to sigma one by one, each term rounded at sigma's size (FP64 3.0e-16 of sigma's norm where this
+// gives 1.4e-16, FP32 1.7e-7 and 4.4e-8).  Three scratch sums are loaded before the first is stored (20 orbitals,
+// 14,000 strings FP64 263 -> 201 ms; 22 orbitals, 16,000 216 -> 172).
 template <typename T, bool kSym, bool kSig>
-__global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T *__restrict__ C, T *__restrict__ sigma) {
+__global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T *__restrict__ C, T *__restrict__ sigma,
+                                                              RowScratch sc) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t slot;
   Bars *bars = reinterpret_cast<Bars *>(smem);
   T *Bs = reinterpret_cast<T *>(smem + sizeof(Bars));
   T *Ps = Bs + (size_t)kStages * a.kcap * kCols;
@@ -141,8 +154,21 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
       tc::mbar_init(addr(bars->p_free[i]), kGatherWarps);
     }
     tc::fence_mbar_init();
+    if constexpr (!kSig) {
+      // there are as many scratch rows as CTAs at a time, so one is free; give up after some rounds all the same
+      uint32_t k = blockIdx.x % sc.slots, tries = 64 * sc.slots;
+      while (atomicCAS(&sc.taken[k], 0u, 1u) != 0u && --tries) k = k + 1 < sc.slots ? k + 1 : 0;
+      __threadfence();
+      slot = tries ? k : sc.slots;
+    }
   }
   __syncthreads();
+  if constexpr (!kSig) {
+    if (slot == sc.slots) {
+      if (threadIdx.x == 0) *reinterpret_cast<volatile int *>(a.err) = 5;
+      return;
+    }
+  }
   // every wait is bounded; an expired one is recorded and its warp leaves (the others' waits for it
   // then expire too)
   auto wait = [&](const uint64_t &b, uint32_t parity, int code) {
@@ -287,8 +313,13 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
     const int gw = warp - kLoadWarp - 1;
     const uint32_t per_group = (uint32_t)a.passes * a.nchunks, steps = ngroups * per_group;
     T *srow = sigma + (size_t)ia * a.nb;
-    if (kSig)
+    T *scr = nullptr;
+    if constexpr (kSig) {
       for (uint32_t c = 32 * gw + lane; c < a.nb; c += 32 * kGatherWarps) sig_s[c] = T(0);
+    } else {
+      scr = reinterpret_cast<T *>(sc.rows) + (size_t)slot * a.nb;
+      for (uint32_t c = 32 * gw + lane; c < a.nb; c += 32 * kGatherWarps) scr[c] = T(0);
+    }
     unsigned char *own = prog_s + 2 * gw * a.prog_cap;
     auto fetch = [&](uint32_t cell, uint32_t s) {
       const uint4 h = a.hdr[cell * kGatherWarps + gw];
@@ -325,6 +356,16 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
       for (uint32_t t = lane; t < ng; t += 32 * kIlp) {
         uint32_t e[kIlp][kRounds];
         T v[kIlp][kRounds];
+        uint32_t gib[kIlp];
+        T gs[kIlp];
+        if constexpr (!kSig) {
+          // (the Ib of a cell's groups are distinct)
+#pragma unroll
+          for (int j = 0; j < kIlp; j++) {
+            gib[j] = t + 32 * j < ng ? ibs[t + 32 * j] : ibs[0];
+            gs[j] = scr[gib[j]];
+          }
+        }
 #pragma unroll
         for (int j = 0; j < kIlp; j++)
 #pragma unroll
@@ -340,8 +381,8 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
           if (t + 32 * j < ng) {
             const uint32_t ib = ibs[t + 32 * j];
             const T sum = (v[j][0] + v[j][1]) + (v[j][2] + v[j][3]);
-            if (kSig) sig_s[ib] += sum;
-            else srow[ib] = (T)((double)srow[ib] + a.scale * (double)sum);
+            if constexpr (kSig) sig_s[ib] += sum;
+            else scr[gib[j]] = gs[j] + sum;
           }
       }
       // the few groups with more entries (the same lane has them)
@@ -357,8 +398,8 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
           }
           const uint32_t ib = ibs[t];
           const T sum = (v[0] + v[1]) + (v[2] + v[3]);
-          if (kSig) sig_s[ib] += sum;
-          else srow[ib] = (T)((double)srow[ib] + a.scale * (double)sum);
+          if constexpr (kSig) sig_s[ib] += sum;
+          else scr[ib] += sum;
         }
       }
       __syncwarp();
@@ -367,9 +408,31 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
     }
     cp_wait<0>();
     __syncwarp();
-    if (kSig)
+    if constexpr (kSig) {
       for (uint32_t c = 32 * gw + lane; c < a.nb; c += 32 * kGatherWarps)
         srow[c] = (T)((double)srow[c] + a.scale * (double)sig_s[c]);
+    } else {
+      for (uint32_t c0 = 32 * gw + lane; c0 < a.nb; c0 += 8 * 32 * kGatherWarps) {
+        T o[8], v[8];  // eight columns' loads side by side
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const uint32_t c = c0 + i * 32 * kGatherWarps;
+          o[i] = c < a.nb ? srow[c] : T(0);
+          v[i] = c < a.nb ? scr[c] : T(0);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const uint32_t c = c0 + i * 32 * kGatherWarps;
+          if (c < a.nb) srow[c] = (T)((double)o[i] + a.scale * (double)v[i]);
+        }
+      }
+      // the three warps are done with the scratch row
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kGatherWarps) : "memory");
+      if (threadIdx.x == 32 * (kLoadWarp + 1)) {
+        __threadfence();
+        atomicExch(&sc.taken[slot], 0u);
+      }
+    }
   }
 }
 
@@ -385,7 +448,12 @@ int launch_rows(sbd_tpb_handle *h, RowArgs a, const T *C, T *sigma) {
   const size_t smem = rows_smem(h->abr, sizeof(T), a.nb, kSig, a.pbufs);
   const auto kern = ab_rows_kernel<T, kSym, kSig>;
   TPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<h->abr.nrows, kThreads, smem, h->stream>>>(a, C, sigma);
+  if constexpr (!kSig) {
+    int ctas = 0;
+    TPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kern, kThreads, smem));
+    if ((uint32_t)(ctas * h->num_sms) > h->abr.slots) return fail(SBD_TPB_ERR_CUDA, "alpha-beta row kernel: scratch rows");
+  }
+  kern<<<h->abr.nrows, kThreads, smem, h->stream>>>(a, C, sigma, RowScratch{h->abr.scratch, h->abr.taken, h->abr.slots});
   TPB_LAUNCHED(h);
   return SBD_TPB_OK;
 }
@@ -566,6 +634,12 @@ static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
   };
   const size_t o_rows = part(rows), o_ent = part(ent), o_pair = part(pair_m), o_m = part(m_pair), o_hdr = part(hdr),
                o_prog = part(prog);
+  // scratch rows where an FP64 row of sums does not fit in shared memory: one CTA of the kernel fills an SM's
+  // registers (512 threads of 128)
+  r.slots = rows_smem(r, sizeof(double), nb, true, 2) > h->smem_optin ? h->num_sms : 0;
+  const std::vector<uint32_t> taken(r.slots, 0);
+  const size_t o_taken = part(taken), o_scratch = bytes;
+  bytes += sizeof(double) * nb * r.slots;
   size_t free_b = 0, total_b = 0;
   TPB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   if (bytes > free_b / 8) return SBD_TPB_OK;
@@ -578,6 +652,7 @@ static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
   TPB_CUDA(place(o_m, m_pair));
   TPB_CUDA(place(o_hdr, hdr));
   TPB_CUDA(place(o_prog, prog));
+  TPB_CUDA(place(o_taken, taken));
   TPB_CUDA(cudaStreamSynchronize(h->stream));
   r.rows = reinterpret_cast<uint32_t *>(d + o_rows);
   r.ent = reinterpret_cast<uint2 *>(d + o_ent);
@@ -585,6 +660,8 @@ static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
   r.m_pair = reinterpret_cast<int32_t *>(d + o_m);
   r.hdr = reinterpret_cast<uint4 *>(d + o_hdr);
   r.prog = d + o_prog;
+  r.taken = reinterpret_cast<uint32_t *>(d + o_taken);
+  r.scratch = d + o_scratch;
   r.err = g_status[h->device % kMaxDevices].get();
   if (!r.err) return fail(SBD_TPB_ERR_OOM, "alpha-beta row program: pinned status word");
   r.ready = true;
@@ -640,7 +717,7 @@ int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym, double scal
   a.prog_cap = r.prog_cap;
   a.scale = scale;
   a.err = r.err;  // unified addressing: the same pointer on the device
-  // the sigma row is summed in shared memory where it fits, else in place
+  // the row is summed in shared memory where it fits, else in a scratch row
   if (rows_smem(r, sizeof(T), a.nb, true, 2) <= h->smem_optin)
     return sym ? launch_rows<T, true, true>(h, a, C, sigma) : launch_rows<T, false, true>(h, a, C, sigma);
   return sym ? launch_rows<T, true, false>(h, a, C, sigma) : launch_rows<T, false, false>(h, a, C, sigma);

@@ -146,6 +146,8 @@ struct ABRows {
   int32_t *pair_m = nullptr, *m_pair = nullptr;  // pair <-> row of the product
   uint4 *hdr = nullptr;
   unsigned char *prog = nullptr;
+  void *scratch = nullptr;  // rows of sums that do not fit in shared memory, and which are in use
+  uint32_t *taken = nullptr, slots = 0;
   int M = 0, passes = 0, bpp = 0;
   uint32_t nrows = 0, nchunks = 0, kcap = 0, prog_cap = 0;
   int *err = nullptr;  // status of the kernel's bounded waits (pinned host memory it writes to)

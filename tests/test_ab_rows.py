@@ -5,12 +5,14 @@ go wrong.
 
 Sets: n strings of lowest orbital-index sum with noise, so that they hold tens of singles each.  Column
 steps are 32 wide, rows of the product come in blocks of 8 (one pass up to 24 blocks), singles in groups
-of 64, and a sigma row that does not fit shared memory is added to in place.
+of 64, and a sigma row that does not fit shared memory is summed in a scratch row.
 """
 import itertools
 
 import numpy as np
 import pytest
+
+from conftest import launched_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -35,6 +37,7 @@ CASES = {
     "union": (18, (7, 1101), (7, 1103)),       # just above the line of the union passes: narrow FP32 tiles
     "many_blocks": (18, (7, 1400), (7, 2101)),  # the widest thread tiles of the same-spin passes, odd rows
     "wide": (18, (7, 24), (7, 15001)),         # a sigma row longer than shared memory holds in FP64
+    "wide_rows": (18, (7, 301), (7, 9001)),    # the same with more rows than SMs
 }
 
 
@@ -95,4 +98,28 @@ def test_alpha_beta_rows_symmetric_half(name, dtype):
     h.sigma_device(x, out, symmetric=True)
     err = float((out.double() - ref.double()).abs().max()) / float(ref.double().abs().max())
     assert err <= (1e-13 if dtype == "float64" else 3e-6), err
+    h.close()
+
+
+def test_wide_rows_lose_no_digits():
+    """A row of sums that does not fit in shared memory (FP32 above some 35,000 columns) is summed from zero
+    as well: the FP32 sigma stays within the rounding of its own result (2^-24 / sqrt(3) = 3.4e-8 of its norm)
+    and of sums of some hundred FP32 terms about as large.  Added to sigma one by one the terms cost 1.7e-7."""
+    import torch
+
+    import sbd_tpb
+    import synth
+    norb, na, nb = 20, 24, 40001
+    h1, eri, core = synth.synthetic_hamiltonian(norb, seed=5)
+    prob = sbd_tpb.Problem(norb=norb, nelec=14, core=core, h1=h1, eri_packed=eri, astr=_dense(norb, 7, na, 1),
+                           bstr=_dense(norb, 7, nb, 1))
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(prob.ndet, dtype=torch.float32, device="cuda", generator=g)
+    y, ref = torch.zeros_like(x), torch.zeros(prob.ndet, dtype=torch.float64, device="cuda")
+    h.sigma_device(x.double(), ref)
+    assert any("ab_rows_kernel" in k for k in launched_kernels(lambda: h.sigma_device(x, y)))
+    err = float((y.double() - ref).norm() / ref.norm())
+    assert err <= 7e-8, err
     h.close()
