@@ -291,7 +291,10 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
       const uint32_t ket0 = lane < kg ? a.a_ent[ge + lane].x : 0, ket1 = lane + 32 < kg ? a.a_ent[ge + 32 + lane].x : 0;
       for (int pass = 0; pass < a.passes; pass++)
         for (uint32_t chunk = 0; chunk < a.nchunks; chunk++, s++) {
-          if (s >= kStages && !wait(bars->c_free[st], ph ^ 1, 3)) return;
+          if (s >= kStages && !wait(bars->c_free[st], ph ^ 1, 3)) {
+            cp_wait<0>();  // the copies in flight
+            return;
+          }
           T *dst = Bs + (size_t)st * a.kcap * kCols;
           const uint32_t col = chunk * kCols + lane;
           const bool cin = col < a.nb;
