@@ -939,26 +939,38 @@ inline bool small_problem(const sbd_tpb_handle *h, size_t nrows, size_t ncols) {
 }
 
 // Whether the union passes are ahead of the per-row ones, from the doubles per distinct ket of a row
-// block (`reuse`), the largest block's table entries and the kind of column access.  The per-row passes
-// stage a block's whole table, so few of their CTAs fit an SM when it is large; the union passes stage
-// 64 kets at a time whatever its size.  At equal residency a per-row pass takes about 0.42 (FP64) and
-// 0.36 to 0.43 (FP32) of a union pass's time per unit of reuse with 16-byte rows, 0.6 with scalar ones; with
-// 3, 2 and 1 CTAs fitting an SM FP64 takes 0.62, 0.88 and 1.6.  The lines are where the products reach 1.
+// block (`reuse`), the largest block's table entries, the kind of column access and the grid.  The per-row
+// passes stage a block's whole table, so few of their CTAs fit an SM when it is large; the union passes
+// stage 64 kets at a time whatever its size.  With four or more CTAs on an SM a per-row pass takes about
+// 0.45 (FP64), 0.43 (FP32; 0.36 one-pass) of a union pass's time per unit of reuse with 16-byte rows, 0.6 with
+// scalar ones; with 3, 2 and 1 CTAs fitting FP64 takes 0.62, 0.88 and 1.6.  The lines are where the products
+// reach 1; two things move them.  Fewer than 256 columns leave threads of a union tile idle: the line
+// of one more CTA, in FP32 two.  And the FP32 general passes' tiles of 8 x 512 may not give an SM four CTAs however many fit.
 // ms of one pass, per row / union (reuse, CTAs that fit): FP64, 16-byte rows: 20 orbitals, 2,000 strings
 // (1.75, 7) 0.40 / 0.47; 22, 6,000 (1.58, 4) 3.7 / 4.6; 26, 16,000 (1.38, 3) 25.2 / 28.3; 20, 6,000 (1.82, 3)
 // 8.6 / 7.7; 24, 16,000 (1.46, 2) 49 / 38; 18 molecular, 4,040 (2.14, 2) 7.7 / 4.3; 26 molecular, 3,900 (2.10, 1)
-// 16.2 / 5.0.  FP32: 20, 6,000 (1.82, 4) 4.7 / 5.6; 22, 16,000 (1.64, 3) sum of both passes 84.5 / 92.9; 18
-// molecular, 4,040 (2.14, 3) 4.2 / 3.1; 18 molecular, 1,388 (2.40, 5) 0.45 / 0.33; 20, 14,000 (1.89, 2) 67.5 / 56.7.
-// Scalar rows, FP64: 22, 4,001 (1.54, 6) 1.44 / 1.61; 22, 6,001 (1.58, 4) 5.3 / 4.7; 24, 8,001 (1.42, 4) sum 12.8 /
-// 11.9; 18 molecular, 4,041 (2.14, 2) 12.1 / 4.3.  FP32: 22, 6,001 (1.58, 6) sum 6.56 / 6.87; 20, 2,001 (1.76, 8)
-// 0.41 / 0.39; 20, 6,001 (1.82, 4) 7.0 / 5.7; 18 molecular, 1,387 (2.40, 5) 0.58 / 0.33.
+// 16.2 / 5.0.  FP32 general: 20, 6,000 (1.82, 4) 4.7 / 5.6; 22, 16,000 (1.64, 3) sum of both passes 84.5 / 92.9; 18
+// molecular, 4,040 (2.14, 3) 4.2 / 3.1; 20, 14,000 (1.89, 2) 67.5 / 56.7; 21 molecular, 1,445 x 1,020 (2.33, 4 but
+// 2.4 CTAs an SM) 0.44 / 0.34; 100 columns: 24, 30,000 (1.50, 2) 2.0 / 2.6.  One-pass: 18 molecular, 4,040 (2.14, 3)
+// 3.23 / 3.09; 1,200 (2.44, 5) 0.26 / 0.30.  Scalar rows, FP64: 22, 4,001 (1.54, 6) 1.44 / 1.61; 22, 6,001 (1.58, 4)
+// 5.3 / 4.7; 24, 8,001 (1.42, 4) sum 12.8 / 11.9; 18 molecular, 4,041 (2.14, 2) 12.1 / 4.3.  FP32: 22, 6,001 (1.58, 6)
+// sum 6.56 / 6.87; 20, 2,001 (1.76, 8) 0.41 / 0.39; 20, 6,001 (1.82, 4) 7.0 / 5.7; 18 molecular, 1,387 (2.40, 5)
+// 0.58 / 0.33.
 template <typename T>
-bool union_ahead(const sbd_tpb_handle *h, double reuse, size_t max_d, size_t max_s, bool rows16) {
+bool union_ahead(const sbd_tpb_handle *h, double reuse, size_t max_d, size_t max_s, size_t nrows, size_t ncols,
+                 bool rows16, bool sym) {
   constexpr int kMost = 5;  // residency beyond which the line stays
-  static constexpr double line[2][2][kMost + 1] = {{{0.0, 1.15, 1.15, 1.15, 1.4, 1.65}, {0.0, 1.15, 1.15, 1.65, 2.1, 2.1}},
-                                                   {{0.0, 1.15, 1.15, 1.15, 1.45, 1.75}, {0.0, 1.5, 1.5, 2.0, 2.35, 2.35}}};
-  const size_t ctas = (h->smem_optin + 1024) / (max_d * (4 + sizeof(T)) + max_s * 16 + 1024);
-  return reuse > 0.0 && reuse >= line[sizeof(T) == 4][rows16][std::min<size_t>(ctas, kMost)];
+  constexpr bool f32 = sizeof(T) == 4;
+  static constexpr double scalar_row[2][kMost + 1] = {{0.0, 1.15, 1.15, 1.15, 1.4, 1.65}, {0.0, 1.15, 1.15, 1.15, 1.45, 1.7}};
+  static constexpr double vector_row[2][kMost + 1] = {{0.0, 1.15, 1.15, 1.65, 2.1, 2.1}, {0.0, 1.5, 1.5, 2.0, 2.35, 2.35}};
+  static constexpr double one_pass32[kMost + 1] = {0.0, 1.5, 1.5, 2.05, 2.75, 2.75};
+  size_t ctas = (h->smem_optin + 1024) / (max_d * (4 + sizeof(T)) + max_s * 16 + 1024);
+  if (rows16 && ctas > 0 && ncols < 256) ctas += f32 ? 2 : 1;
+  const size_t c = std::min<size_t>(ctas, kMost);
+  double line = !rows16 ? scalar_row[f32][c] : f32 && sym ? one_pass32[c] : vector_row[f32][c];
+  if (rows16 && f32 && !sym && (nrows + kBlkRows - 1) / kBlkRows * ((ncols + 511) / 512) < 4 * (size_t)h->num_sms)
+    line = std::min(line, 1.55);
+  return reuse > 0.0 && reuse >= line;
 }
 
 // Launch shapes of the general passes.  16-byte rows without the alpha-single x beta-single terms
@@ -1101,13 +1113,14 @@ __global__ void __launch_bounds__(256)
 // Shared memory of union_fill_kernel: a byte of rows and the place in the list per ket.
 inline size_t union_map_bytes(size_t n) { return (n + 3) / 4 * 4 + n * 4; }
 
-// The entries of a sigma program's union list (n strings, max_d / max_s: its largest block), built on
-// first use per problem and type; left out (u->off null) where the per-row passes are ahead or it would
+// The entries of a sigma program's union list (n strings, max_d / max_s: its largest block; ncols columns of
+// the other spin), built on first use per problem and type; left out (u->off null) where the per-row passes are ahead or it would
 // take more than an eighth of the free memory.
 template <typename T>
-int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, size_t max_d, size_t max_s, bool rows16, UnionArgs *u) {
+int build_union(sbd_tpb_handle *h, SigmaProg &p, size_t n, size_t max_d, size_t max_s, size_t ncols, bool rows16, bool sym,
+                UnionArgs *u) {
   *u = UnionArgs();
-  if (!p.u_off || !union_ahead<T>(h, p.u_reuse, max_d, max_s, rows16)) return SBD_TPB_OK;
+  if (!p.u_off || !union_ahead<T>(h, p.u_reuse, max_d, max_s, n, ncols, rows16, sym)) return SBD_TPB_OK;
   T **val = reinterpret_cast<T **>(sizeof(T) == 8 ? (void **)&p.u_val : (void **)&p.u_valf);
   if (!*val) {
     const size_t bytes = sizeof(T) * kBlkRows * p.u_total;
@@ -1394,9 +1407,10 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
     const uint32_t *m = h->blk_max;
     // (the union passes read the singles' Coulomb sums from their table)
     if (h->pa.jtab || !h->ta_s.nnz)
-      TPB_CHECK(build_union<T>(h, h->pa, na, m[0], m[1], rows_aligned(nb, C, sigma, CT), &ua));
+      TPB_CHECK(build_union<T>(h, h->pa, na, m[0], m[1], nb, rows_aligned(nb, C, sigma, CT), false, &ua));
     if (h->pb.jtab || !h->tb_s.nnz)
-      TPB_CHECK(build_union<T>(h, h->same_strings ? h->pa : h->pb, nb, m[2], m[3], rows_aligned(na, CT, sigma), &ub));
+      TPB_CHECK(build_union<T>(h, h->same_strings ? h->pa : h->pb, nb, m[2], m[3], na, rows_aligned(na, CT, sigma), false,
+                               &ub));
   }
 
   BlockArgs ba{};
@@ -1490,7 +1504,7 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   UnionArgs ua;
   if (!small_problem(h, na, nb) && (h->pa.jtab || !h->ta_s.nnz))
-    TPB_CHECK(build_union<T>(h, h->pa, na, h->blk_max[0], h->blk_max[1], rows_aligned(nb, C, sigma), &ua));
+    TPB_CHECK(build_union<T>(h, h->pa, na, h->blk_max[0], h->blk_max[1], nb, rows_aligned(nb, C, sigma), true, &ua));
   BlockArgs ba{};
   ba.u = ua;
   ba.s_off = h->ta_s.off;

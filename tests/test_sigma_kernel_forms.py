@@ -94,7 +94,7 @@ def test_aligned_and_offset_vectors_give_same_bits(name, dtype):
     (24, 8, 1500, "float64", False),  # 1.29
     (24, 8, 1501, "float32", False),
 ])
-def test_union_passes_run_where_they_are_ahead(norb, ne, count, dtype, union):
+def test_union_passes_on_sampled_sets(norb, ne, count, dtype, union):
     """On sampled sets the per-row passes with 16-byte rows stay ahead well above 1.5 doubles per distinct
     ket (20 orbitals, 2,000 strings: FP64 0.39 against 0.46 ms, FP32 0.23 against 0.36)."""
     import torch
@@ -108,4 +108,35 @@ def test_union_passes_run_where_they_are_ahead(norb, ne, count, dtype, union):
     for symmetric in (False, True):
         ran = _passes(launched_kernels(lambda: h.sigma_device(x, y, symmetric=symmetric)))
         assert ran and all(("sigma_union_kernel" in k) == union for k in ran), ran
+    h.close()
+
+
+@pytest.mark.parametrize("norb, ne, na, nb, dtype, symmetric, alpha, beta", [
+    # a grid of 2.4 CTAs an SM: FP32 union passes from 1.55 doubles per distinct ket (0.34 against 0.44 ms)
+    (21, 5, 1444, 1020, "float32", False, True, True),
+    # beta's 8,000 rows of 100 columns: threads of a union tile idle (FP32 1.04 against 1.16 ms at 160)
+    (20, 6, 100, 14000, "float32", False, False, False),
+    (20, 6, 100, 14000, "float64", False, False, True),
+    # one-pass FP32 at 2.4 doubles per distinct ket: 0.26 against 0.30 ms
+    (18, 7, 1200, 1200, "float32", True, False, None),
+    (18, 7, 1200, 1200, "float64", True, True, None),
+])
+def test_union_passes_on_rectangular_and_one_pass(norb, ne, na, nb, dtype, symmetric, alpha, beta):
+    import torch
+
+    import sbd_tpb
+    import synth
+    from test_ab_rows import _dense
+    h1, eri, core = synth.synthetic_hamiltonian(norb)
+    strings = [synth.sample_strings(norb, ne, n) if (norb, ne) == (20, 6) else _dense(norb, ne, n, 1) for n in (na, nb)]
+    prob = sbd_tpb.Problem(norb=norb, nelec=2 * ne, core=core, h1=h1, eri_packed=eri, astr=strings[0], bstr=strings[1])
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    x = torch.randn(na, nb, dtype=getattr(torch, dtype), device="cuda")
+    if symmetric:
+        x = x + x.T
+    x = x.reshape(-1).contiguous()
+    y = torch.zeros_like(x)
+    ran = ["union" in k for k in _passes(launched_kernels(lambda: h.sigma_device(x, y, symmetric=symmetric)))]
+    assert ran == ([alpha] if symmetric else [alpha, beta])
     h.close()
