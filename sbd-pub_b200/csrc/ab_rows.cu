@@ -66,7 +66,6 @@ struct RowArgs {
   uint32_t pbufs;         // buffers of P
   uint32_t kcap;          // rows of the staged C block (a multiple of 8, at most kMaxK)
   uint32_t prog_cap;      // bytes of one program buffer
-  double scale;
   int *err;               // pinned host memory: set when a wait expired
 };
 
@@ -413,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
     __syncwarp();
     if constexpr (kSig) {
       for (uint32_t c = 32 * gw + lane; c < a.nb; c += 32 * kGatherWarps)
-        srow[c] = (T)((double)srow[c] + a.scale * (double)sig_s[c]);
+        srow[c] = (T)((double)srow[c] + (double)sig_s[c]);
     } else {
       for (uint32_t c0 = 32 * gw + lane; c0 < a.nb; c0 += 8 * 32 * kGatherWarps) {
         T o[8], v[8];  // eight columns' loads side by side
@@ -426,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) ab_rows_kernel(RowArgs a, const T
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const uint32_t c = c0 + i * 32 * kGatherWarps;
-          if (c < a.nb) srow[c] = (T)((double)o[i] + a.scale * (double)v[i]);
+          if (c < a.nb) srow[c] = (T)((double)o[i] + (double)v[i]);
         }
       }
       // the three warps are done with the scratch row
@@ -699,7 +698,7 @@ int ab_rows_check(sbd_tpb_handle *h) {
 // sigma += the alpha-beta terms.  sym (identical string lists, C = C^T): only the half B of the terms
 // whose transposes are the others, so that B + B^T is the whole term.
 template <typename T>
-int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym, double scale) {
+int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym) {
   const ABRows &r = h->abr;
   RowArgs a{};
   a.rows = r.rows;
@@ -718,7 +717,6 @@ int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym, double scal
   a.nb = (uint32_t)h->bstr.size();
   a.kcap = r.kcap;
   a.prog_cap = r.prog_cap;
-  a.scale = scale;
   a.err = r.err;  // unified addressing: the same pointer on the device
   // the row is summed in shared memory where it fits, else in a scratch row
   if (rows_smem(r, sizeof(T), a.nb, true, 2) <= h->smem_optin)
@@ -726,7 +724,7 @@ int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym, double scal
   return sym ? launch_rows<T, true, false>(h, a, C, sigma) : launch_rows<T, false, false>(h, a, C, sigma);
 }
 
-template int ab_rows_apply<double>(sbd_tpb_handle *, const double *, double *, bool, double);
-template int ab_rows_apply<float>(sbd_tpb_handle *, const float *, float *, bool, double);
+template int ab_rows_apply<double>(sbd_tpb_handle *, const double *, double *, bool);
+template int ab_rows_apply<float>(sbd_tpb_handle *, const float *, float *, bool);
 
 }  // namespace sbdtpb

@@ -290,7 +290,7 @@ int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host);
 void ab_rows_free(sbd_tpb_handle *h);
 int ab_rows_check(sbd_tpb_handle *h);  // status of the launches before the last synchronisation
 template <typename T>
-int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym, double scale = 1.0);
+int ab_rows_apply(sbd_tpb_handle *h, const T *C, T *sigma, bool sym);
 // vecops.cu
 int ensure_partials(sbd_tpb_handle *h, size_t n);
 template <typename T>
