@@ -16,6 +16,7 @@
 // tensor pipe instead of through two shared-memory reads each.
 #include <algorithm>
 #include <bitset>
+#include <cmath>
 #include <mutex>
 #include <new>
 #include <string>
@@ -508,9 +509,20 @@ void ab_rows_free(sbd_tpb_handle *h) {
   r = ABRows();
 }
 
-// The row program; ready stays false where the direct kernel is the better one or the program does not fit.
-static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
+// Which kernel: the multiply-adds of the products (padded) over those of the direct loop, which does each of
+// them through two shared-memory reads.  The rows kernel runs up to these ratios.  Direct / rows time, FP64
+// general, symmetric, FP32 general, symmetric: 26 orbitals, 120 molecular strings (ratio 10) 4.1, 4.1, 3.4, 3.8; 18
+// orbitals, 4,041 (4) 4.1, 3.9, 3.2, 3.1; sampled strings: 20 orbitals, 6,000 (10) 2.6, 2.4, 2.1, 1.9; 21, 6,000 (14.9)
+// 1.8, 1.6, 1.1, 1.0; 20, 3,500 (16.7) 1.37, 1.32, 1.10, 1.06; 22, 13,000 (17.1) 1.93, 1.64, 1.21, 1.07; 22, 11,000
+// (19.8) 1.57, 1.34, 1.04, 0.92; 20, 3,000 (19.9) 1.14, 1.06, 0.94, 0.88; 20, 2,700 (22.6) 0.92, 0.87, 0.78, 0.73; 22,
+// 8,000 (26.6) 1.07, 0.92, 0.71, 0.63.  Sets with one or two singles a string lie above 100, where the padded
+// products lose tenfold.  FP32 has the lower line: its vectors pay FP64 products.
+constexpr double kMostRatio64 = 20.0, kMostRatio32 = 17.0;
+
+// The row program where the ratio is at most `most`; ready stays false where it is not or the program does not fit.
+static int build_program(sbd_tpb_handle *h, SinglesHost &host, double most) {
   ABRows &r = h->abr;
+  r.ratio = HUGE_VAL;
   const size_t na = h->astr.size(), nb = h->bstr.size(), L2 = (size_t)h->L * h->L;
   const size_t nnza = h->ta_s.nnz, nnzb = h->tb_s.nnz;
   if (!nnza || !nnzb) return SBD_TPB_OK;
@@ -533,11 +545,6 @@ static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
   r.passes = (blocks + kMaxBlocks - 1) / kMaxBlocks;
   r.bpp = (blocks + r.passes - 1) / r.passes;
   r.nchunks = (uint32_t)((nb + kCols - 1) / kCols);
-  // Which kernel: multiply-adds of the products (padded) against those of the direct loop, which does
-  // each of them through two shared-memory reads.  Ratio 18 (18 orbitals, 150 strings, 12 singles a
-  // string): 0.034 against 0.098 ms; ratio 4 (4,041 strings): 12.6 against 50.9; 20 orbitals, 6,000 sampled
-  // strings (a few singles, ratio about 15) 15.9 against 27.0.  Selected sets with one or two singles
-  // a string lie above 100, where the padded products lose.
   double gemm = 0.0;
   uint32_t kmax = 0;
   for (size_t i = 0; i < na; i++) {
@@ -545,8 +552,8 @@ static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
     kmax = std::max(kmax, k);
     gemm += (double)((k + 7) / 8 * 8);
   }
-  gemm *= 8.0 * r.bpp * r.passes * (double)nb;
-  if (gemm > 20.0 * (double)nnza * (double)nnzb) return SBD_TPB_OK;
+  r.ratio = gemm * 8.0 * r.bpp * r.passes * (double)nb / ((double)nnza * (double)nnzb);
+  if (r.ratio > most) return SBD_TPB_OK;
   std::vector<uint32_t> rows;
   for (size_t i = 0; i < na; i++)
     if (ao[i + 1] > ao[i]) rows.push_back((uint32_t)i);
@@ -670,18 +677,23 @@ static int build_program(sbd_tpb_handle *h, SinglesHost &host) {
   return SBD_TPB_OK;
 }
 
-// Builds the program once per problem.  Memory that runs short, the host's or the device's, leaves the direct
-// kernel to do the term.
-int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host) {
-  if (h->abr.tried) return SBD_TPB_OK;
+// Whether the term of this type's vectors takes the rows kernel; the program is built once per problem, when the
+// first type takes it.  Memory that runs short, the host's or the device's, leaves the direct kernel to do the term.
+int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host, bool f32, bool *use) {
+  const double most = f32 ? kMostRatio32 : kMostRatio64;
+  *use = h->abr.ready && h->abr.ratio <= most;
+  if (h->abr.tried || h->abr.ratio > most) return SBD_TPB_OK;  // (ratio 0: not counted yet)
   int rc;
   try {
-    rc = build_program(h, host);
+    rc = build_program(h, host, most);
   } catch (const std::bad_alloc &) {
     rc = SBD_TPB_ERR_OOM;
   }
+  const double ratio = h->abr.ratio;
   if (!h->abr.ready) ab_rows_free(h);
-  h->abr.tried = true;
+  h->abr.ratio = ratio;
+  h->abr.tried = ratio <= most;
+  *use = h->abr.ready;
   if (rc != SBD_TPB_ERR_OOM) return rc;
   cudaGetLastError();
   return SBD_TPB_OK;

@@ -1396,8 +1396,8 @@ int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, dou
   }
   T *CT = reinterpret_cast<T *>(h->d_ct);
   SinglesHost host;
-  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h, host));
-  const bool rows_ab = h->abr.ready && !dense_ab;
+  bool rows_ab = false;
+  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h, host, sizeof(T) == 4, &rows_ab));
   TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab, host));
   // per-pair Coulomb sums of the singles over the other spin's strings (built once per problem)
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
@@ -1498,8 +1498,8 @@ int sigma_sep_sym(sbd_tpb_handle *h, const T *C, T *sigma, double shift, const T
     return fail(SBD_TPB_ERR_STATE, "symmetric sigma needs identical alpha and beta strings");
   const bool dense_ab = h->ab.enabled && sizeof(T) == 4 && h->ab.tc_ready;
   SinglesHost host;
-  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h, host));
-  const bool rows_ab = h->abr.ready && !dense_ab;
+  bool rows_ab = false;
+  if (!dense_ab) TPB_CHECK(ab_rows_prepare(h, host, sizeof(T) == 4, &rows_ab));
   TPB_CHECK(prepare_sigma_meta(h, !rows_ab && !dense_ab, host));
   TPB_CHECK(build_coulomb_table(h, h->pa, h->d_bstr, nb));
   UnionArgs ua;

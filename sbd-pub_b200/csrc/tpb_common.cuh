@@ -140,6 +140,7 @@ struct ABDense {
 // blocks of ket columns, and the alpha singles in the order the symmetric form needs.
 struct ABRows {
   bool tried = false, ready = false;
+  double ratio = 0.0;                            // multiply-adds against the direct kernel's; 0: not counted
   unsigned char *block = nullptr;                // the one allocation that the arrays below lie in
   uint32_t *rows = nullptr;                      // alpha rows with singles, most singles first
   uint2 *ent = nullptr;                          // alpha singles (ket, +-(pair + 1))
@@ -286,7 +287,7 @@ bool ab_dense_worthwhile(sbd_tpb_handle *h);
 template <typename T>
 int ab_dense_apply(sbd_tpb_handle *h, const T *C, T *sigma, double scale = 1.0);
 // ab_rows.cu: alpha-beta term of densely connected sets, one tensor-core product per alpha row
-int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host);
+int ab_rows_prepare(sbd_tpb_handle *h, SinglesHost &host, bool f32, bool *use);
 void ab_rows_free(sbd_tpb_handle *h);
 int ab_rows_check(sbd_tpb_handle *h);  // status of the launches before the last synchronisation
 template <typename T>

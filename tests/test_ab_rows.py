@@ -123,3 +123,29 @@ def test_wide_rows_lose_no_digits():
     err = float((y.double() - ref).norm() / ref.norm())
     assert err <= 7e-8, err
     h.close()
+
+
+@pytest.mark.parametrize("first", ["float64", "float32"])
+def test_the_line_is_lower_for_fp32(first):
+    """Sampled strings at a ratio of 18.5 multiply-adds to the direct kernel's: FP64 takes the rows kernel (1.2 times
+    as fast), FP32, whose vectors pay FP64 products too, the direct one -- whichever asks first."""
+    import torch
+
+    import sbd_tpb
+    import synth
+    h1, eri, core = synth.synthetic_hamiltonian(20)
+    s = synth.sample_strings(20, 6, 2800)
+    prob = sbd_tpb.Problem(norb=20, nelec=12, core=core, h1=h1, eri_packed=eri, astr=s, bstr=s.copy())
+    h = sbd_tpb.Handle(0)
+    h.set_problem(prob)
+    x = torch.from_numpy(np.random.default_rng(1).normal(size=prob.ndet)).cuda()
+    out = {}
+    for dtype in (first, "float32" if first == "float64" else "float64"):
+        v = x.to(getattr(torch, dtype))
+        out[dtype] = torch.zeros_like(v)
+        ran = launched_kernels(lambda: h.sigma_device(v, out[dtype]))
+        assert any(("ab_rows" if dtype == "float64" else "ab_sparse") in k for k in ran), ran
+    # FP32: vectors and results rounded to FP32, 2^-24 a value over a few thousand terms of random sign
+    diff = (out["float32"].double() - out["float64"]).abs().max() / out["float64"].abs().max()
+    assert float(diff) <= 2e-6
+    h.close()
