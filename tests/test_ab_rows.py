@@ -25,6 +25,8 @@ def _dense(norb, n, count, seed):
     return np.sort((np.int64(1) << idx[keep]).sum(axis=1).astype(np.uint64))
 
 
+SMS = 148
+
 CASES = {
     # norb, (alpha electrons, strings), (beta electrons, strings): what is at its edge
     "full8": (8, (4, 70), (4, 70)),            # 28 pairs: the last block of 8 rows half empty
@@ -36,6 +38,8 @@ CASES = {
     "one_row": (10, (5, 2), (5, 252)),         # rows with a single single
     "union": (18, (7, 1101), (7, 1103)),       # just above the line of the union passes: narrow FP32 tiles
     "many_blocks": (18, (7, 1400), (7, 2101)),  # the widest thread tiles of the same-spin passes, odd rows
+    "union_sym": (18, (7, 1400), (7, 1400)),   # the one-pass form on the union passes (FP64)
+    "two_passes_sym": (24, (5, 1301), (5, 1301)),  # 276 pairs, two passes, each with its triangle of the terms
     "wide": (18, (7, 24), (7, 15001)),         # a sigma row longer than shared memory holds in FP64
     "wide_rows": (18, (7, 301), (7, 9001)),    # the same with more rows than SMs
 }
@@ -67,6 +71,9 @@ def test_alpha_beta_rows_against_oracle(name):
     x = rng.normal(size=prob.ndet)
     rows = np.sort(rng.choice(prob.ndet, size=min(300, prob.ndet), replace=False)).astype(np.uint64)
     ref = _oracle_rows(prob, x, rows)
+    ran = launched_kernels(lambda: h.sigma(x))
+    assert any("ab_rows_kernel" in k for k in ran)
+    assert any("sigma_union_kernel" in k for k in ran) == (prob.ndet >= 8192 * SMS)
     out = h.sigma(x)
     assert np.array_equal(out, h.sigma(x))  # one owner per element: the same bits again
     scale = float(np.max(np.abs(ref)))
@@ -95,7 +102,10 @@ def test_alpha_beta_rows_symmetric_half(name, dtype):
     ref, out = torch.zeros_like(x), torch.full_like(x, float("nan"))
     torch.cuda.synchronize()  # the library runs on a stream of its own
     h.sigma_device(x, ref)
-    h.sigma_device(x, out, symmetric=True)
+    ran = launched_kernels(lambda: h.sigma_device(x, out, symmetric=True))
+    if dtype == "float64":
+        assert any("ab_rows_kernel" in k for k in ran)
+        assert any("sigma_union_kernel" in k for k in ran) == (prob.ndet >= 8192 * SMS)
     err = float((out.double() - ref.double()).abs().max()) / float(ref.double().abs().max())
     assert err <= (1e-13 if dtype == "float64" else 3e-6), err
     h.close()
