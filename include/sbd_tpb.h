@@ -300,8 +300,9 @@ SBD_TPB_API void *sbd_tpb_stream(sbd_tpb_handle *h);
 SBD_TPB_API double sbd_tpb_last_sigma_ms(sbd_tpb_handle *h);
 
 /* Per-stage device times (ms) of the last sigma call, in launch order: [0] alpha pass (diagonal,
- * alpha singles/doubles, C^T), [1] beta pass, [2] alpha-beta term (sparse kernel or dense
- * gather/contract/scatter).  Returns how many were written (<= max_n) or a negative status. */
+ * alpha singles/doubles, C^T), [1] beta pass, [2] alpha-beta term (direct kernel, one product per
+ * alpha row, or gather/contract/scatter); in convention 2 [0] the one-pass alpha pass, [1] the alpha-beta
+ * term, [2] the transpose-add; sbd_tpb_sigma_noalloc has [0] and [1] only.  Returns how many were written (<= max_n) or a negative status. */
 SBD_TPB_API int sbd_tpb_last_sigma_kernels(sbd_tpb_handle *h, double *ms, int max_n);
 
 /* Number of kernel launches the library has issued on this handle (for accounting). */

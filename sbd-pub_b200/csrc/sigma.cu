@@ -5,16 +5,18 @@
 // FP64 atomics, every sigma element here has exactly one owner, so results are deterministic:
 //
 //   alpha pass    sigma[Ia, Ib] = (H_ii - shift) C[Ia, Ib] + sum_Ja H_a(Ia, Ja) C[Ja, Ib]
-//                 (+ the alpha-single x beta-single terms sa sb (pq|rs) C[Ja, Jb] when the
-//                 singles are sparse), gathering rows Ja of C from an L2-resident column slab;
+//                 (+ the alpha-single x beta-single terms sa sb (pq|rs) C[Ja, Jb] in the
+//                 allocation-free form), gathering rows Ja of C from an L2-resident column slab;
 //                 the same CTA writes its own tile of C transposed into C^T.
 //   beta pass     sigma[Ia, Ib] += sum_Jb H_b(Ib, Jb) C^T[Jb, Ia], the same kernel on C^T, its
 //                 result transposed back through shared memory with coalesced writes.
 // Both passes are the alpha-string "row SpMM" on a row-major operand, which is what makes every
 // gather a 128-byte coalesced row segment.
 //
-// The alpha-beta term of FCI-like problems (dense singles) goes through the gather -> dense
-// (pq|rs) contraction -> scatter path in ab_dense.cu instead of the direct loop.
+// On densely connected sets both passes share kets between rows (sigma_union.cuh).  The alpha-beta term has three
+// kernels: ab_sparse_kernel here, the direct loop, where singles are sparse; one FP64 tensor-core product per
+// alpha row (ab_rows.cu) where they are dense; and for FP32 vectors of FCI-like problems gather -> dense (pq|rs)
+// contraction -> scatter on tcgen05 (ab_dense.cu, ab_tc.cu).
 #include <algorithm>
 #include <string>
 
@@ -35,9 +37,10 @@ constexpr int kBlkThreads = 128;
 // 2/8: 3.66 / 1.52, 1/6/OS: 3.77 / 1.50, 2/9/OS spills: 3.84 / 1.78); FP32 beta 2/8 3.35 / 1.36 /
 // 0.159 (2/9: 3.38 / 1.44 / 0.185, 2/10: 3.68 / 1.63, 4/10: 14.4); FP64 alpha 2/7 6.39 / 2.53 /
 // 0.187 (2/8: 6.44, 2/7/OS: 6.45, 2/6: 6.95); FP64 beta 2/9 5.76 / 2.71 / 0.196 (2/8: 5.93 / 2.38 /
-// 0.197, 2/10: 6.09).  Four groups lose the 16-byte runs of the FP32 transposed write-out.  Small
-// problems run the FP32 alpha pass with 2/6 and no parking (norb=12 FCI 0.154 ms; 2/7: 0.159,
-// 2/7/OS: 0.161, 2/8/OS: 0.170, 1/5: 0.279); the switch is at 10,000 one-group CTAs.
+// 0.197, 2/10: 6.09).  Four groups lose the 16-byte runs of the FP32 transposed write-out.  Below 10,000
+// one-group CTAs the FP32 alpha pass runs with 2/6 and no parking (norb=12 FCI 0.154 ms; 2/7: 0.159,
+// 2/7/OS: 0.161, 2/8/OS: 0.170, 1/5: 0.279).  The 12-orbital figures were taken with these shapes; a problem of that
+// size now takes one row per thread (small_problem).
 // The mapping of a pass as template arguments: G row groups, register budget of M CTAs per SM.
 template <typename T>
 __device__ __forceinline__ T val_of(const double *v, const float *vf, uint32_t e);
@@ -1381,7 +1384,7 @@ template <typename T>
 int sigma_sep_shift(sbd_tpb_handle *h, const T *C, T *sigma, int accumulate, double shift) {
   const uint32_t na = (uint32_t)h->astr.size(), nb = (uint32_t)h->bstr.size();
   // Alpha-beta term: densely connected sets take one product per alpha row (ab_rows.cu; when, see
-  // ab_rows_prepare), except small FP32 problems, whose gather / contraction / scatter on tcgen05 is
+  // kMostRatio64 there), except small FP32 problems, whose gather / contraction / scatter on tcgen05 is
   // still ahead at full-CI connectivity (norb=12 FCI symmetric 0.341 against 0.354 ms); in FP64 the
   // CUDA-core form of that path loses to both others (3.4 ms there).  Sparse singles take the direct
   // kernel.

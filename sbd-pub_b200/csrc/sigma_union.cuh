@@ -8,7 +8,9 @@
 // then its singles, with sigma_block_kernel's arithmetic: the same bits.
 //
 // A thread's VW columns lie 128 apart, so every access of a warp is one contiguous run whatever the
-// row length; VW is chosen by the number of CTAs (launch_union).  Bound by issue slots and L2 gathers.
+// row length; VW is chosen by the number of CTAs (launch_union).  Bound by the gathers' round trips to L2: half
+// of a warp's cycles between two issues, with 19 warps an SM (88 registers in FP64); L1/TEX is 66 % busy, the
+// issue slots 53 %, the FP64 pipe 36 %, L2 36 %.  When these passes are taken: union_ahead.
 // ms per pass, per-row kernels -> here: 18 orbitals, 4,041 strings (odd rows) FP64 alpha 11.9 -> 4.3, beta
 // 12.5 -> 4.3; 24 orbitals, 5,514 strings FP32 one-pass 19.8 -> 8.0; 18 orbitals, 1,387 strings FP64 0.86 /
 // 0.91 -> 0.47 / 0.49, FP32 0.72 / 0.76 -> 0.33 / 0.35.
