@@ -59,7 +59,7 @@ struct RowArgs {
   const int32_t *pair_m;  // pair pq -> row of P of its unordered pair, -1 when no beta single has it
   const int32_t *m_pair;  // row of P -> pair
   const uint4 *hdr;       // per (pass, chunk, gather warp): (byte offset of its program, groups, rounds, byte offset of its entries)
-  const unsigned char *prog;  // first entry of each round, Ib of each group, entries (see ab_rows_prepare)
+  const unsigned char *prog;  // first entry of each round, Ib of each group, entries (see build_program)
   const double *eri;
   int L2, M;
   int passes, bpp;        // passes over the rows of P, 8-row blocks per pass
