@@ -948,11 +948,12 @@ inline bool small_problem(const sbd_tpb_handle *h, size_t nrows, size_t ncols) {
 // 0.45 (FP64), 0.43 (FP32; 0.36 one-pass) of a union pass's time per unit of reuse with 16-byte rows, 0.6 with
 // scalar ones; with 3, 2 and 1 CTAs fitting FP64 takes 0.62, 0.88 and 1.6.  The lines are where the products
 // reach 1; two things move them.  Fewer than 256 columns leave threads of a union tile idle: the line
-// of one more CTA, in FP32 two.  And the FP32 general passes' tiles of 8 x 512 may not give an SM four CTAs however many fit.
+// of one more CTA, in FP32 two.  And just above the line of the one-row passes the tiles (8 x 512, FP64 8 x
+// 256) give an SM too few CTAs however many fit: 1.6 where FP32 has fewer than 4 an SM, FP64 fewer than 5 1/4.
 // ms of one pass, per row / union (reuse, CTAs that fit): FP64, 16-byte rows: 20 orbitals, 2,000 strings
 // (1.75, 7) 0.40 / 0.47; 22, 6,000 (1.58, 4) 3.7 / 4.6; 26, 16,000 (1.38, 3) 25.2 / 28.3; 20, 6,000 (1.82, 3)
 // 8.6 / 7.7; 24, 16,000 (1.46, 2) 49 / 38; 18 molecular, 4,040 (2.14, 2) 7.7 / 4.3; 26 molecular, 3,900 (2.10, 1)
-// 16.2 / 5.0.  FP32 general: 20, 6,000 (1.82, 4) 4.7 / 5.6; 22, 16,000 (1.64, 3) sum of both passes 84.5 / 92.9; 18
+// 16.2 / 5.0; 20, 1,200 (1.71, 8 but 5.1 CTAs an SM) 0.165 / 0.148.  FP32 general: 20, 6,000 (1.82, 4) 4.7 / 5.6; 22, 16,000 (1.64, 3) sum of both passes 84.5 / 92.9; 18
 // molecular, 4,040 (2.14, 3) 4.2 / 3.1; 20, 14,000 (1.89, 2) 67.5 / 56.7; 21 molecular, 1,445 x 1,020 (2.33, 4 but
 // 2.4 CTAs an SM) 0.44 / 0.34; 100 columns: 24, 30,000 (1.50, 2) 2.0 / 2.6.  One-pass: 18 molecular, 4,040 (2.14, 3)
 // 3.23 / 3.09; 1,200 (2.44, 5) 0.26 / 0.30.  Scalar rows, FP64: 22, 4,001 (1.54, 6) 1.44 / 1.61; 22, 6,001 (1.58, 4)
@@ -971,8 +972,8 @@ bool union_ahead(const sbd_tpb_handle *h, double reuse, size_t max_d, size_t max
   if (rows16 && ctas > 0 && ncols < 256) ctas += f32 ? 2 : 1;
   const size_t c = std::min<size_t>(ctas, kMost);
   double line = !rows16 ? scalar_row[f32][c] : f32 && sym ? one_pass32[c] : vector_row[f32][c];
-  if (rows16 && f32 && !sym && (nrows + kBlkRows - 1) / kBlkRows * ((ncols + 511) / 512) < 4 * (size_t)h->num_sms)
-    line = std::min(line, 1.55);
+  const size_t tile = f32 ? 512 : 256, grid = (nrows + kBlkRows - 1) / kBlkRows * ((ncols + tile - 1) / tile);
+  if (rows16 && !(f32 && sym) && 4 * grid < (f32 ? 16 : 21) * (size_t)h->num_sms) line = std::min(line, 1.6);
   return reuse > 0.0 && reuse >= line;
 }
 

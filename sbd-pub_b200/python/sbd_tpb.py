@@ -315,7 +315,8 @@ class Handle:
         return lib().sbd_tpb_last_sigma_ms(self.h)
 
     def last_sigma_kernels(self):
-        """Device ms of each stage of the last sigma: [alpha pass, beta pass, alpha-beta term]."""
+        """Device ms of each stage of the last sigma: [alpha pass, beta pass, alpha-beta term], or in the symmetric
+        form [one-pass alpha pass, alpha-beta term, transpose-add]."""
         buf = (C.c_double * 8)()
         n = lib().sbd_tpb_last_sigma_kernels(self.h, buf, 8)
         _check(n if n < 0 else OK)

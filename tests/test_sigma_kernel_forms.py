@@ -112,9 +112,10 @@ def test_union_passes_on_sampled_sets(norb, ne, count, dtype, union):
 
 
 @pytest.mark.parametrize("norb, ne, na, nb, dtype, symmetric, alpha, beta", [
-    # a grid of 2.4 CTAs an SM: FP32 union passes from 1.55 doubles per distinct ket (0.34 against 0.44 ms)
+    # a grid of 2.4 CTAs an SM: FP32 union passes from 1.6 doubles per distinct ket (0.34 against 0.44 ms)
     (21, 5, 1444, 1020, "float32", False, True, True),
-    # beta's 8,000 rows of 100 columns: threads of a union tile idle (FP32 1.04 against 1.16 ms at 160)
+    (20, 6, 1200, 1200, "float64", False, True, True),  # 5.1 CTAs an SM, 1.7 doubles per distinct ket
+    # beta's 14,000 rows of 100 columns: threads of a union tile idle (FP32 2.0 against 2.6 ms at 30,000)
     (20, 6, 100, 14000, "float32", False, False, False),
     (20, 6, 100, 14000, "float64", False, False, True),
     # one-pass FP32 at 2.4 doubles per distinct ket: 0.26 against 0.30 ms
